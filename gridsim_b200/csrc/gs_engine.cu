@@ -76,9 +76,12 @@ __device__ __forceinline__ bool zipLoad(const DevGrid& g, int i, double vm, doub
 //    replaced by their reduced values), the mismatch into the right-hand side (and its FP64 copy in mixed
 //    precision), the Jacobian blocks of row i into their LU slots; folds |mismatch| into localMax and sets bad
 //    (1: mismatch not finite, 2: Jacobian not finite).
-template <typename T>
+// LG lanes share a bus (aligned groups of a warp, all of them here together): its cells dealt to them in turn, the sums
+// completed over the group; the first lane does the rest.
+template <typename T, int LG = 1>
 __device__ __forceinline__ void busMismatchJac(const DevGrid& g, const DevBatch& b, int i, int s, int fillJac, double* pOut,
                                                double* qOut, double& localMax, int& bad) {
+    const int gl = LG == 1 ? 0 : (int)(threadIdx.x & (LG - 1));
     const size_t B = (size_t)b.B;
     const double vmi = b.vm[i * B + s], vai = b.va[i * B + s];
     // Grids analysed with every bus's P and Q rows (qlim): the bus's type in this system (3 reference, 2 PV, 1 PQ,
@@ -91,16 +94,19 @@ __device__ __forceinline__ void busMismatchJac(const DevGrid& g, const DevBatch&
     const bool qId = g.qlim && et != 1;
     const int kp = g.busP[i], kq = g.busQ[i];
     const bool fill = fillJac && (kp >= 0 || kq >= 0);
-    T* lu = (T*)b.lu;
+    const size_t K = b.own ? 1 : B;  // the Jacobian and right-hand side: interleaved, or this system's own
+    const int so = b.own ? 0 : s;
+    T* lu = (T*)b.lu + so;
     // one pass over row i: the injections, and the off-diagonal Jacobian blocks from the same sin/cos (they do not
     // need P, Q); the diagonal blocks follow from the sums
     double pi = 0.0, qi = 0.0, Gd = 0.0, Bd = 0.0;
     int pd = -1;
     const int p0 = g.yRowPtr[i], p1 = g.yRowPtr[i + 1];
     CellOverride ovr(g, b.outage[s], p0);
-    for (int p = p0; p < p1; p++) {
+    for (int p = p0 + gl; p < p1; p += LG) {
         const int j = g.yCol[p];
         double G = g.yG[p], Bv = g.yB[p];
+        if (LG > 1) ovr.seek(p);
         ovr.at(g, p, G, Bv);
         double sn, cs;
         sincos(vai - b.va[j * B + s], &sn, &cs);
@@ -114,11 +120,23 @@ __device__ __forceinline__ void busMismatchJac(const DevGrid& g, const DevBatch&
         const double M = qId ? 0.0 : -vmi * vmj * (G * cs + Bv * sn);
         const double L = qId ? 0.0 : vmi * (G * sn - Bv * cs);
         const int4 sl = *reinterpret_cast<const int4*>(g.ySlot + 4 * p);
-        if (sl.x >= 0) lu[sl.x * B + s] = (T)H;
-        if (sl.y >= 0) lu[sl.y * B + s] = (T)N;
-        if (sl.z >= 0) lu[sl.z * B + s] = (T)M;
-        if (sl.w >= 0) lu[sl.w * B + s] = (T)L;
+        if (sl.x >= 0) lu[sl.x * K] = (T)H;
+        if (sl.y >= 0) lu[sl.y * K] = (T)N;
+        if (sl.z >= 0) lu[sl.z * K] = (T)M;
+        if (sl.w >= 0) lu[sl.w * K] = (T)L;
         bad |= (isfinite(H) && isfinite(N) && isfinite(M) && isfinite(L)) ? 0 : 2;
+    }
+    if (LG > 1) {
+        const unsigned mask = ((1u << LG) - 1u) << (threadIdx.x & 31 & ~(LG - 1));
+#pragma unroll
+        for (int o = LG / 2; o > 0; o >>= 1) {
+            pi += __shfl_xor_sync(mask, pi, o);
+            qi += __shfl_xor_sync(mask, qi, o);
+            Gd += __shfl_xor_sync(mask, Gd, o);
+            Bd += __shfl_xor_sync(mask, Bd, o);
+            pd = max(pd, __shfl_xor_sync(mask, pd, o));
+        }
+        if (gl != 0) return;
     }
     const double P = vmi * pi, Q = vmi * qi;
     const double sc = b.loadScale ? b.loadScale[i * B + s] : 1.0;
@@ -133,10 +151,10 @@ __device__ __forceinline__ void busMismatchJac(const DevGrid& g, const DevBatch&
         const double M = qId ? 0.0 : P - Gd * vmi * vmi;
         const double L = qId ? 1.0 : Q / vmi - Bd * vmi + (vcol ? zdQdV : 0.0);
         const int4 sl = *reinterpret_cast<const int4*>(g.ySlot + 4 * pd);
-        if (sl.x >= 0) lu[sl.x * B + s] = (T)H;
-        if (sl.y >= 0) lu[sl.y * B + s] = (T)N;
-        if (sl.z >= 0) lu[sl.z * B + s] = (T)M;
-        if (sl.w >= 0) lu[sl.w * B + s] = (T)L;
+        if (sl.x >= 0) lu[sl.x * K] = (T)H;
+        if (sl.y >= 0) lu[sl.y * K] = (T)N;
+        if (sl.z >= 0) lu[sl.z * K] = (T)M;
+        if (sl.w >= 0) lu[sl.w * K] = (T)L;
         bad |= (isfinite(H) && isfinite(N) && isfinite(M) && isfinite(L)) ? 0 : 2;
     }
     if (pOut) { pOut[i * B + s] = P; qOut[i * B + s] = Q; }
@@ -150,23 +168,23 @@ __device__ __forceinline__ void busMismatchJac(const DevGrid& g, const DevBatch&
         if (gt == 2) b.qinj[i * B + s] = Q;
         if (et == 1 && gt != 1) qspec = b.qspecSys[i * B + s];
     }
-    T* y = (T*)b.y;
+    T* y = (T*)b.y + so;
     if (kp >= 0 && pId) {
-        y[kp * B + s] = T(0);
+        y[kp * K] = T(0);
         if (b.rhs64) b.rhs64[kp * B + s] = 0.0;
     } else if (kp >= 0) {
         const double f = pspec - P - zdP;
-        y[kp * B + s] = (T)f;
+        y[kp * K] = (T)f;
         if (b.rhs64) b.rhs64[kp * B + s] = f;
         localMax = fmax(localMax, fabs(f));
         bad |= isfinite(f) ? 0 : 1;
     }
     if (kq >= 0 && qId) {
-        y[kq * B + s] = T(0);
+        y[kq * K] = T(0);
         if (b.rhs64) b.rhs64[kq * B + s] = 0.0;
     } else if (kq >= 0) {
         const double f = qspec - Q - zdQ;
-        y[kq * B + s] = (T)f;
+        y[kq * K] = (T)f;
         if (b.rhs64) b.rhs64[kq * B + s] = f;
         localMax = fmax(localMax, fabs(f));
         bad |= isfinite(f) ? 0 : 1;
@@ -263,9 +281,7 @@ constexpr double kRevertVoltTolPu = 1e-4;   // NewtonShell.cs:31
 constexpr int kMaxQPasses = 100;            // PowerFlowOptions.MaxQLimitPasses default (:101)
 enum : int32_t { kQReverted = 16 };
 
-__global__ void k_status_q(DevBatch b, double tol, double divLimit, int maxIter) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= b.count || !b.active[s]) return;
+__device__ __forceinline__ void statusQStep(const DevBatch& b, int s, double tol, double divLimit, int maxIter) {
     b.qState[s] &= ~kQSkipStep;
     const int iter = b.passIter[s];
     const double mis = __longlong_as_double((long long)b.maxMis[s]);
@@ -298,6 +314,11 @@ __global__ void k_status_q(DevBatch b, double tol, double divLimit, int maxIter)
     atomicAdd(b.activeCount, 1);
 }
 
+__global__ void k_status_q(DevBatch b, double tol, double divLimit, int maxIter) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s < b.count && b.active[s]) statusQStep(b, s, tol, divLimit, maxIter);
+}
+
 // TryRevertPin (NewtonShell.cs:563-576): a bus pinned at a limit whose voltage crossed its set point (by 1e-4 pu, on
 // the side the limit pushes it) goes back to PV at the set point, once per solve.
 __device__ __forceinline__ bool tryRevertPin(const DevGrid& g, const DevBatch& b, int i, int s, size_t idx) {
@@ -315,10 +336,9 @@ __device__ __forceinline__ bool tryRevertPin(const DevGrid& g, const DevBatch& b
     return true;
 }
 
-// ApplyQLimits on the systems whose pass converged: grid (ceil(n / 8), B / 32), block (32, 8).
-__global__ void k_qapply(DevGrid g, DevBatch b) {
-    const int s = blockIdx.y * 32 + threadIdx.x, i = blockIdx.x * 8 + threadIdx.y;
-    if (!g.qlimOn || i >= g.n || s >= b.count || !b.active[s] || !(b.qState[s] & kQPending) || g.busType[i] != 2) return;
+// ApplyQLimits on bus i of a system whose pass converged.
+__device__ __forceinline__ void qApplyBus(const DevGrid& g, const DevBatch& b, int i, int s) {
+    if (!g.qlimOn || g.busType[i] != 2) return;
     const size_t idx = (size_t)i * b.B + s;
     if (b.effType[idx] != 2) {  // with RevertQLimits a pinned bus may go back to PV in the same pass (:551-556)
         if (g.qlimRevert && tryRevertPin(g, b, i, s, idx)) atomicOr(&b.qState[s], kQChanged);
@@ -345,22 +365,29 @@ __global__ void k_qapply(DevGrid g, DevBatch b) {
         atomicOr(&b.qState[s], kQChanged);
     }
 }
-
-// RevertBrokenPins on the systems whose pass converged without a switch.
-__global__ void k_qrevert(DevGrid g, DevBatch b) {
+// grid (ceil(n / 8), B / 32), block (32, 8)
+__global__ void k_qapply(DevGrid g, DevBatch b) {
     const int s = blockIdx.y * 32 + threadIdx.x, i = blockIdx.x * 8 + threadIdx.y;
-    if (i >= g.n || s >= b.count || !b.active[s] || g.busType[i] != 2) return;
-    const int st = b.qState[s];
+    if (i < g.n && s < b.count && b.active[s] && (b.qState[s] & kQPending)) qApplyBus(g, b, i, s);
+}
+
+// RevertBrokenPins on bus i of a system whose pass converged without a switch. (The state word is changed by atomics of
+// the other threads of the pass: read past L1.)
+__device__ __forceinline__ void qRevertBus(const DevGrid& g, const DevBatch& b, int i, int s) {
+    if (g.busType[i] != 2) return;
+    const int st = __ldcg(b.qState + s);
     if (!(st & kQPending) || (st & kQChanged)) return;
     const size_t idx = (size_t)i * b.B + s;
     if (tryRevertPin(g, b, i, s, idx)) atomicOr(&b.qState[s], kQReverted);
 }
+__global__ void k_qrevert(DevGrid g, DevBatch b) {
+    const int s = blockIdx.y * 32 + threadIdx.x, i = blockIdx.x * 8 + threadIdx.y;
+    if (i < g.n && s < b.count && b.active[s]) qRevertBus(g, b, i, s);
+}
 
 // The end of a converged pass: a switch starts the next pass (this iteration's step is not taken), else converged.
-__global__ void k_qfinish(DevBatch b, int maxPasses) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= b.count || !b.active[s]) return;
-    const int st = b.qState[s];
+__device__ __forceinline__ void qFinishStep(const DevBatch& b, int s, int maxPasses) {
+    const int st = __ldcg(b.qState + s);
     if (!(st & kQPending)) return;
     if (st & (kQChanged | kQReverted)) {
         b.qPass[s] += 1;
@@ -373,6 +400,10 @@ __global__ void k_qfinish(DevBatch b, int maxPasses) {
         b.active[s] = 0;
         b.qState[s] = 0;
     }
+}
+__global__ void k_qfinish(DevBatch b, int maxPasses) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s < b.count && b.active[s]) qFinishStep(b, s, maxPasses);
 }
 
 // Systems admitted at different times (the request loop): each at its own step count. Systems that stop
@@ -1456,6 +1487,10 @@ __global__ void k_init(DevGrid g, DevBatch b, const double* vmStart, const doubl
     }
 }
 
+}  // namespace gs
+#include "gs_solo.cuh"
+namespace gs {
+
 // ---------------------------------------------------------------------------------------------
 // Post-processing of converged systems (ContingencyAnalysis.ScreenStateCore :1150-1235): branch
 // loading (NewtonShell.ComputeLineFlows :699-734), the thermal test (> 100 %), the voltage test against
@@ -1718,6 +1753,7 @@ struct gs_ctx {
     std::map<std::string, int> multiTune;  // the multi-grid batch's CTA shape per set of grids (autotuned)
     std::vector<std::unique_ptr<MatrixPattern>> patterns;  // most recently used last
     unsigned long long* noallocScratch = nullptr;  // device address of the allocation-free check's static scratch
+    int sms = 148;
     bool clusterOk = false;  // the few-systems cluster walk can be scheduled on this device
     ~gs_ctx();
 };
@@ -1739,6 +1775,8 @@ struct gs_grid {
     gs::DevBuf setBrBuf, setCellBuf, setRedBuf;
     int split = 0;      // first level run by the persistent kernels (factorisation)
     int splitB = 0;     // first level run by the persistent kernels in the triangular solves
+    gs::DevSolo solo{};  // one block's shared-memory program of the grid, where its factors fit (on)
+    gs::DevBuf soloNext; // its system counter and step maximum (calls on the context's stream)
     int tailSplit = 0;  // first level the few-systems path runs as one CTA per system
     int tailMax = gs::kTailMaxSystems;  // the few-systems path takes over at this many systems still stepping
     int psSplit = 0, psSplitB = 0;      // the same first persistent levels on the paired schedule
@@ -1979,6 +2017,15 @@ int UploadGrid(gs_grid* G) {
         UP(P.factor.levelWide, pfWide); UP(P.backward.levelWide, pbWide); UP(P.forward.levelWide, pvWide);
         UP(P.factor.levelMid, pfMid); UP(P.backward.levelMid, pbMid); UP(P.forward.levelMid, pvMid);
         v.psLevels = P.nLevels;
+    }
+    G->solo.on = 0;
+    if (const SoloProgram S = BuildSolo(s); S.on && std::getenv("GS_NO_SOLO") == nullptr) {
+        DevSolo& d = G->solo;
+        std::vector<int4> chunks(S.chunks.size() / 4);
+        std::memcpy(chunks.data(), S.chunks.data(), S.chunks.size() * 4);
+        if ((rc = Upload(G, chunks, &d.chunks)) != GS_OK || (rc = Upload(G, S.first, &d.first)) != GS_OK) return rc;
+        d.m = S.m; d.nVal = S.nVal; d.yBase = S.yBase; d.zero = S.zero; d.one = S.one;
+        d.on = 1;
     }
 #undef UP
     // the few-systems path runs the lowest levels as per-level launches while a phase of them holds more short
@@ -2252,6 +2299,32 @@ int Newton(gs_grid* G, int count, bool useScale, bool startFromWs, const gs_pf_o
     k_init<<<dim3((s.n + 7) / 8, groups), blk8, 0, st>>>(g, b, startFromWs ? w.startVm.as<double>() : nullptr,
                                                           startFromWs ? w.startVa.as<double>() : nullptr, vmSys, vaSys);
     GS_CUDA(cudaGetLastError());
+    // with Q limits every pass may take up to max_iterations steps (plus the step-less pass switches)
+    const int maxLoop = g.qlim ? (o.max_iterations + 2) * (g.qlimMaxPasses + 2) : o.max_iterations + 4;
+    if (G->solo.on && !G->gpMode && o.phase_timing == 0) {
+        // the factors fit a block's shared memory: every system's whole run in one launch
+        const DevSolo& P = G->solo;
+        const size_t smem = SoloSmem(P.nVal, P.m);
+        int occ = 0;
+        GS_CUDA(G->soloNext.alloc(2 * sizeof(int)));
+        GS_CUDA(cudaMemsetAsync(G->soloNext.p, 0, 2 * sizeof(int), st));
+        GS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_solo, kSoloThreads, smem));
+        k_solo<<<std::min(count, std::max(1, occ) * ctx->sms), kSoloThreads, smem, st>>>(
+            g, P, b, G->soloNext.as<int>(), o.tolerance, o.diverge_limit_pu, o.max_iterations, maxLoop, G->soloNext.as<int>() + 1);
+        GS_CUDA(cudaGetLastError());
+        cudaMemcpyAsync(ctx->pinnedCount, G->soloNext.as<int>() + 1, sizeof(int), cudaMemcpyDeviceToHost, st);
+        cudaEventRecord(e1, st);
+        const cudaError_t se = cudaEventSynchronize(e1);
+        if (se == cudaSuccess && ms) cudaEventElapsedTime(ms, e0, e1);
+        cudaEventDestroy(e0);
+        cudaEventDestroy(e1);
+        if (se != cudaSuccess) return SetErr(ctx, GS_ERR_CUDA, std::string("newton: ") + cudaGetErrorString(se));
+        if (stats) {
+            stats->launches += 2;
+            stats->iterations = std::max(stats->iterations, *ctx->pinnedCount);
+        }
+        return GS_OK;
+    }
     // the step (factor levels, backward levels, refinement, max |dx|, update) as one graph
     const int refine = sizeof(T) < sizeof(double) ? 1 : 0;
     const bool timed = o.phase_timing != 0;
@@ -2456,8 +2529,6 @@ int Newton(gs_grid* G, int count, bool useScale, bool startFromWs, const gs_pf_o
     bool compacted = false;
     bool midOn = false;  // cur is the mid workspace (its origin list maps it back to b)
     const dim3 nodeBlocks((s.n + 7) / 8);
-    // with Q limits every pass may take up to max_iterations steps (plus the step-less pass switches)
-    const int maxLoop = g.qlim ? (o.max_iterations + 2) * (g.qlimMaxPasses + 2) : o.max_iterations + 4;
     for (int iter = 0; iter <= maxLoop; iter++) {
         if (timed) cudaEventRecord(ev[0], st);
         if (listCount > 0)
@@ -3099,6 +3170,7 @@ int gs_ctx_create(int device, const gs_ctx_opts* opts, gs_ctx** out) {
     if (cudaSetDevice(device) != cudaSuccess || gs::SetKernelAttributes() != cudaSuccess ||
         cudaStreamCreateWithFlags(&c->partStream[1], cudaStreamNonBlocking) != cudaSuccess) { delete c; return GS_ERR_CUDA; }
     if (cudaMallocHost(&c->pinnedCount, 4 * sizeof(int)) != cudaSuccess) { delete c; return GS_ERR_CUDA; }
+    cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device);
     c->clusterOk = gs::ClusterWalkAvailable() && std::getenv("GS_NO_CLUSTER_TAIL") == nullptr;
     *out = c;
     return GS_OK;
@@ -4246,6 +4318,8 @@ cudaError_t SetKernelAttributes() {
     set((const void*)k_tail<double, kWorkForward>);
     set((const void*)k_newton<float>);
     set((const void*)k_newton<double>);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute((const void*)k_solo, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSoloSmemMax);
     return e;
 }
 }  // namespace gs

@@ -182,6 +182,40 @@ struct SubtreeSchedule {
 };
 SubtreeSchedule BuildSubtrees(const Symbolic& s, int cut);
 
+// The program of one system's linear solve (factorisation with the fused forward substitution, then the backward
+// substitution) held in a block's shared memory (gs_solo.cuh). Its values: the LU slots of Symbolic (node-major), the
+// right-hand side from yBase, a zero, a scratch value; beside them the reciprocal pivots, and a one. L and U are kept undivided, A = L D^-1 U,
+// so that every entry of a level (diagonal, row, column, right-hand side) is one sum over values of lower levels,
+// out - sum L(a) dinv(j) U(c), and a level takes one barrier.
+// A level is cut into bundles of 32 / G sums, G lanes a sum, a lane's share of the pairs in chunks of kSoloRounds. A warp
+// runs its stream of chunks; a chunk is kSoloRounds quads of words for each of the 32 lanes (quad k of all lanes, then
+// quad k + 1): {a, c, j} of the lane's k-th pair and one of: the value the sum is taken from, where the result goes, the
+// head, the factor of a backward sum. All but the head are byte offsets from the values (the reciprocal pivots follow
+// them), so that an operand costs no more than its load. Unused pairs read the zero; lanes without a result to store
+// (unused ones, and all but the first of a sum's) store into a scratch value.
+// head: the lane's kind | log2 G << 4 | kSoloLast (the bundle's sums are complete) | kSoloHasDiag | kSoloIsBack |
+// barriers << 12: the level's end and the levels after it without work for this warp, 0 when the warp has more of the
+// level. Stream of warp w: first[3 w] its first chunk, first[3 w + 1] their number, first[3 w + 2] the levels it waits out
+// before the first one.
+enum SoloKind : int32_t { kSoloEntry = 0, kSoloDiag = 1, kSoloBack = 2, kSoloNone = 3 };
+constexpr int kSoloRounds = 4, kSoloWords = 32 * 4 * kSoloRounds;  // words of a chunk
+constexpr int32_t kSoloLast = 1 << 8, kSoloHasDiag = 1 << 9, kSoloIsBack = 1 << 10;
+constexpr int kSoloWarps = 8;  // warps that run a program
+constexpr int kSoloSlots = 3;  // chunks of a warp's ring in shared memory
+constexpr size_t kSoloSmemMax = 226 * 1024;
+// Dynamic shared memory of the kernel: the values, the reciprocal pivots and a one, the warps' rings.
+inline size_t SoloSmem(int64_t nVal, int m) {
+    return ((size_t)nVal + m + 2) / 2 * 16 + (size_t)kSoloWarps * kSoloSlots * kSoloWords * 4;
+}
+struct SoloPair { int a, c, j; };
+struct SoloProgram {
+    bool on = false;
+    int m = 0, nVal = 0, yBase = 0, zero = 0, one = 0, levels = 0;  // zero (then the scratch): values; one: a reciprocal pivot
+    std::vector<int32_t> chunks, first;
+};
+// The program of s; on = false when its values do not fit a block's shared memory in FP64.
+SoloProgram BuildSolo(const Symbolic& s);
+
 // Build s.top[which] for values of `elem` bytes within `budget` bytes of shared memory.
 void BuildTopPart(Symbolic& s, int which, size_t elem, size_t budget);
 

@@ -162,6 +162,7 @@ struct DevBatch {
     int B;                  // interleave stride (multiple of 32)
     int count;              // live systems
     int nLevels;            // elimination-tree levels of the grid
+    int own;                // lu and y are one system's own arrays (k_solo), not interleaved; the rest is
     double* vm;             // [n][B]
     double* va;             // [n][B]
     void* lu;               // [nnzLU][B] of the LU type (diagonal slots keep A(k, k))
@@ -226,6 +227,11 @@ struct CellOverride {
         } else if (o >= 0) {
             c0 = g.brCell[4 * o]; c1 = g.brCell[4 * o + 1]; c2 = g.brCell[4 * o + 2]; c3 = g.brCell[4 * o + 3];
         }
+    }
+    // move on to cell p (cells in between left out)
+    __device__ __forceinline__ void seek(int p) {
+        if (sc)
+            while (sc[ov] < p) ov++;
     }
     __device__ __forceinline__ void at(const DevGrid& g, int p, double& G, double& Bv) {
         if (p == c0) { G = g.brRed[8 * o + 0]; Bv = g.brRed[8 * o + 1]; }

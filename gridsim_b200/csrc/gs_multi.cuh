@@ -35,30 +35,6 @@ struct SlotArena {
     size_t offLu, offPiv, offY, offZ, offRhs, offVm, offVa, offScal;
 };
 
-__device__ __forceinline__ double blockMaxD(double v, double* red) {
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, off));
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    const int nw = (blockDim.x + 31) >> 5;
-    double r = red[0];
-    for (int k = 1; k < nw; k++) r = fmax(r, red[k]);
-    return r;
-}
-
-__device__ __forceinline__ int blockOrI(int v, int* red) {
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v |= __shfl_xor_sync(0xffffffffu, v, off);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    const int nw = (blockDim.x + 31) >> 5;
-    int r = 0;
-    for (int k = 0; k < nw; k++) r |= red[k];
-    return r;
-}
-
 template <typename T>
 __global__ void __launch_bounds__(1024) k_newton(const DevGrid* grids, const MultiItem* items, int nItems, int* next,
                                                  SlotArena arena, const double* loadScale, const int* outage,

@@ -1,0 +1,46 @@
+"""Newton runs held in one block's shared memory (k_solo) on a B200, through the C ABI: the smallest grid, one of odd
+size, the largest that fit and the first that does not, plain and under StudyOptions (Q-limit passes in the kernel),
+against the oracle on the same inputs: statuses, iterations and violations identical, converged voltages within the
+parity bar of 1e-8 pu and 1e-8 rad."""
+import numpy as np
+import pytest
+
+import oracle
+from gridsim_b200 import _abi, synthetic
+from gridsim_b200.engine import ContingencyAnalysis, PowerFlowOptions, SparseNewtonRaphsonPowerFlow, study_options
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("study", [False, True])
+@pytest.mark.parametrize("n_bus", [6, 31, 120, 640, 1000])
+def test_screens_match_the_oracle(n_bus, study):
+    m = synthetic.make_grid(n_bus, n_bus + n_bus // 3 + 1, max(1, n_bus // 8), seed=3)
+    idx = m.in_service_branches()[:33]
+    opt = study_options("fp64") if study else PowerFlowOptions(max_iterations=20, warm_start_from_base=True)
+    if study:  # limits that bind on some units, so that passes switch buses
+        m.qmin, m.qmax = m.qmin * 0.1, m.qmax * 0.1
+    ref = oracle.screen(m, idx, opt.to_c(), keep_states=True)
+    got = ContingencyAnalysis.screen_raw(m, idx, SparseNewtonRaphsonPowerFlow("fp64"), opt, keep_states=True)
+    assert (got["status"] == ref["status"]).all()
+    assert (got["iterations"] == ref["iterations"]).all()
+    assert (got["viol_ptr"] == ref["viol_ptr"]).all()
+    ok = np.nonzero((ref["status"] == _abi.PF_CONVERGED) & ~synthetic.bridges(m)[idx])[0]
+    assert len(ok)
+    vm, va = np.asarray(ref["vm"]).reshape(len(idx), -1), np.asarray(ref["va_deg"]).reshape(len(idx), -1)
+    assert np.abs(got["vm"][ok] - vm[ok]).max() <= 1e-8
+    assert np.radians(np.abs(got["va_deg"][ok] - va[ok])).max() <= 1e-8
+
+
+@pytest.mark.parametrize("count", [1, 37, 400])
+def test_batches_of_more_systems_than_blocks(count):
+    m = synthetic.make_grid(57, 80, 7, seed=9)
+    scale = np.random.default_rng(1).uniform(0.95, 1.05, size=(count, m.n_bus))
+    opt = PowerFlowOptions(max_iterations=20)
+    got = SparseNewtonRaphsonPowerFlow("fp64").solve_batch(m, load_scale=scale, options=opt, keep_states=True)
+    for k in {0, count // 2, count - 1}:
+        one = m.copy()
+        one.pd, one.qd = m.pd * scale[k], m.qd * scale[k]
+        ref = oracle.solve(one, opt.to_c())
+        assert got["status"][k] == ref["status"] and got["iterations"][k] == ref["iterations"]
+        assert np.abs(got["vm"][k] - ref["vm"]).max() <= 1e-8
