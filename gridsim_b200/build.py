@@ -11,7 +11,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 SRC = [os.path.join(HERE, "csrc", f) for f in ("gs_engine.cu", "gs_host.cpp", "gs_symbolic.cpp", "gs_dc.cpp",
                                                 "gs_topology.cpp", "gs_solo.cpp")]
 OUT = os.path.join(HERE, "libgridsim_b200.so")
-DEPS = SRC + [os.path.join(HERE, "csrc", f) for f in ("gs_internal.h", "gs_host.h", "gs_kernels.cuh", "gs_multi.cuh", "gs_serve.cuh", "gs_cluster.cuh", "gs_paired.cuh", "gs_pivot.cuh", "gs_solo.cuh")] + [
+DEPS = SRC + [os.path.join(HERE, "csrc", f) for f in ("gs_internal.h", "gs_host.h", "gs_kernels.cuh", "gs_multi.cuh", "gs_serve.cuh", "gs_cluster.cuh", "gs_paired.cuh", "gs_pivot.cuh", "gs_solo.cuh", "gs_shared.cuh")] + [
     os.path.join(os.path.dirname(HERE), "include", "gridsim_b200.h")]
 
 
@@ -26,7 +26,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if not force and os.path.exists(OUT) and all(os.path.getmtime(OUT) >= os.path.getmtime(d) for d in DEPS):
         return OUT
     cmd = [nvcc(), "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3",
-           "-split-compile=0", "-Xcompiler", "-fPIC", "-shared", "-o", OUT] + SRC
+           "-Xcompiler", "-fPIC", "-shared", "-o", OUT] + SRC
     if verbose:
         cmd.insert(1, "-Xptxas=-v")
     subprocess.check_call(cmd)

@@ -76,9 +76,9 @@ __device__ __forceinline__ bool zipLoad(const DevGrid& g, int i, double vm, doub
 //    replaced by their reduced values), the mismatch into the right-hand side (and its FP64 copy in mixed
 //    precision), the Jacobian blocks of row i into their LU slots; folds |mismatch| into localMax and sets bad
 //    (1: mismatch not finite, 2: Jacobian not finite).
-// LG lanes share a bus (aligned groups of a warp, all of them here together): its cells dealt to them in turn, the sums
+// OWN: lu and y are one system's own, not interleaved (k_solo). LG lanes share a bus (aligned groups of a warp, all of them here together): its cells dealt to them in turn, the sums
 // completed over the group; the first lane does the rest.
-template <typename T, int LG = 1>
+template <typename T, int LG = 1, bool OWN = false>
 __device__ __forceinline__ void busMismatchJac(const DevGrid& g, const DevBatch& b, int i, int s, int fillJac, double* pOut,
                                                double* qOut, double& localMax, int& bad) {
     const int gl = LG == 1 ? 0 : (int)(threadIdx.x & (LG - 1));
@@ -94,9 +94,9 @@ __device__ __forceinline__ void busMismatchJac(const DevGrid& g, const DevBatch&
     const bool qId = g.qlim && et != 1;
     const int kp = g.busP[i], kq = g.busQ[i];
     const bool fill = fillJac && (kp >= 0 || kq >= 0);
-    const size_t K = b.own ? 1 : B;  // the Jacobian and right-hand side: interleaved, or this system's own
-    const int so = b.own ? 0 : s;
-    T* lu = (T*)b.lu + so;
+    const size_t K = OWN ? 1 : B;  // the Jacobian and right-hand side: interleaved, or this system's own arrays
+    const size_t so = OWN ? 0 : s;
+    T* lu = (T*)b.lu;
     // one pass over row i: the injections, and the off-diagonal Jacobian blocks from the same sin/cos (they do not
     // need P, Q); the diagonal blocks follow from the sums
     double pi = 0.0, qi = 0.0, Gd = 0.0, Bd = 0.0;
@@ -120,10 +120,10 @@ __device__ __forceinline__ void busMismatchJac(const DevGrid& g, const DevBatch&
         const double M = qId ? 0.0 : -vmi * vmj * (G * cs + Bv * sn);
         const double L = qId ? 0.0 : vmi * (G * sn - Bv * cs);
         const int4 sl = *reinterpret_cast<const int4*>(g.ySlot + 4 * p);
-        if (sl.x >= 0) lu[sl.x * K] = (T)H;
-        if (sl.y >= 0) lu[sl.y * K] = (T)N;
-        if (sl.z >= 0) lu[sl.z * K] = (T)M;
-        if (sl.w >= 0) lu[sl.w * K] = (T)L;
+        if (sl.x >= 0) lu[sl.x * K + so] = (T)H;
+        if (sl.y >= 0) lu[sl.y * K + so] = (T)N;
+        if (sl.z >= 0) lu[sl.z * K + so] = (T)M;
+        if (sl.w >= 0) lu[sl.w * K + so] = (T)L;
         bad |= (isfinite(H) && isfinite(N) && isfinite(M) && isfinite(L)) ? 0 : 2;
     }
     if (LG > 1) {
@@ -151,10 +151,10 @@ __device__ __forceinline__ void busMismatchJac(const DevGrid& g, const DevBatch&
         const double M = qId ? 0.0 : P - Gd * vmi * vmi;
         const double L = qId ? 1.0 : Q / vmi - Bd * vmi + (vcol ? zdQdV : 0.0);
         const int4 sl = *reinterpret_cast<const int4*>(g.ySlot + 4 * pd);
-        if (sl.x >= 0) lu[sl.x * K] = (T)H;
-        if (sl.y >= 0) lu[sl.y * K] = (T)N;
-        if (sl.z >= 0) lu[sl.z * K] = (T)M;
-        if (sl.w >= 0) lu[sl.w * K] = (T)L;
+        if (sl.x >= 0) lu[sl.x * K + so] = (T)H;
+        if (sl.y >= 0) lu[sl.y * K + so] = (T)N;
+        if (sl.z >= 0) lu[sl.z * K + so] = (T)M;
+        if (sl.w >= 0) lu[sl.w * K + so] = (T)L;
         bad |= (isfinite(H) && isfinite(N) && isfinite(M) && isfinite(L)) ? 0 : 2;
     }
     if (pOut) { pOut[i * B + s] = P; qOut[i * B + s] = Q; }
@@ -168,23 +168,23 @@ __device__ __forceinline__ void busMismatchJac(const DevGrid& g, const DevBatch&
         if (gt == 2) b.qinj[i * B + s] = Q;
         if (et == 1 && gt != 1) qspec = b.qspecSys[i * B + s];
     }
-    T* y = (T*)b.y + so;
+    T* y = (T*)b.y;
     if (kp >= 0 && pId) {
-        y[kp * K] = T(0);
+        y[kp * K + so] = T(0);
         if (b.rhs64) b.rhs64[kp * B + s] = 0.0;
     } else if (kp >= 0) {
         const double f = pspec - P - zdP;
-        y[kp * K] = (T)f;
+        y[kp * K + so] = (T)f;
         if (b.rhs64) b.rhs64[kp * B + s] = f;
         localMax = fmax(localMax, fabs(f));
         bad |= isfinite(f) ? 0 : 1;
     }
     if (kq >= 0 && qId) {
-        y[kq * K] = T(0);
+        y[kq * K + so] = T(0);
         if (b.rhs64) b.rhs64[kq * B + s] = 0.0;
     } else if (kq >= 0) {
         const double f = qspec - Q - zdQ;
-        y[kq * K] = (T)f;
+        y[kq * K + so] = (T)f;
         if (b.rhs64) b.rhs64[kq * B + s] = f;
         localMax = fmax(localMax, fabs(f));
         bad |= isfinite(f) ? 0 : 1;
@@ -1489,6 +1489,7 @@ __global__ void k_init(DevGrid g, DevBatch b, const double* vmStart, const doubl
 
 }  // namespace gs
 #include "gs_solo.cuh"
+#include "gs_shared.cuh"
 namespace gs {
 
 // ---------------------------------------------------------------------------------------------
@@ -1618,10 +1619,71 @@ __global__ void k_compact(DevGrid g, DevBatch b, Classify c, const int* chunkOff
 }
 
 // Line flows of system 0 (single solve result).
-__global__ void k_lineflows(DevGrid g, DevBatch b, double base, double* loading, double* sfo, double* sto) {
+// rows[k * n + i] (a system a row) into the batch's interleaved[i * B + k] and back times f; systems past cnt are 1.
+// Tiles of 32 x 32 through shared memory, so that both sides move whole lines: grid (ceil(n / 32), ceil(B / 32)), block
+// (32, 8). The host's own transposition of the load scales and states of 777 systems of 2,750 buses took half the call.
+__global__ void k_rows_in(const double* __restrict__ rows, double* __restrict__ out, int n, int B, int cnt) {
+    __shared__ double t[32][33];
+    const int i0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
+    for (int r = threadIdx.y; r < 32; r += 8) {
+        const int k = k0 + r, i = i0 + threadIdx.x;
+        t[r][threadIdx.x] = k < cnt && i < n ? rows[(size_t)k * n + i] : 1.0;
+    }
+    __syncthreads();
+    for (int r = threadIdx.y; r < 32; r += 8) {
+        const int i = i0 + r, k = k0 + threadIdx.x;
+        if (i < n && k < B) out[(size_t)i * B + k] = t[threadIdx.x][r];
+    }
+}
+__global__ void k_rows_out(const double* __restrict__ in, double* __restrict__ rows, int n, int B, int cnt, double f) {
+    __shared__ double t[32][33];
+    const int i0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
+    for (int r = threadIdx.y; r < 32; r += 8) {
+        const int i = i0 + r, k = k0 + threadIdx.x;
+        if (i < n && k < cnt) t[r][threadIdx.x] = in[(size_t)i * B + k];
+    }
+    __syncthreads();
+    for (int r = threadIdx.y; r < 32; r += 8) {
+        const int k = k0 + r, i = i0 + threadIdx.x;
+        if (i < n && k < cnt) rows[(size_t)k * n + i] = t[threadIdx.x][r] * f;
+    }
+}
+
+// System 0's state and control words (status, steps when the tolerance was met, steps, mismatch) gathered.
+__global__ void k_take_base(DevBatch b, int n, double* vm, double* va, double* out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) { vm[i] = b.vm[(size_t)i * b.B]; va[i] = b.va[(size_t)i * b.B]; }
+    if (i == 0) { out[0] = b.status[0]; out[1] = b.convIters[0]; out[2] = b.iters[0]; out[3] = b.finalMis[0]; }
+}
+
+// A single solve's results (system 0) packed as [n] magnitudes, [n] angles in degrees, [n] injections in MW, [n] in MVAr
+// (pq), then the branches' loadings [nbr] and flows [2 nbr], [2 nbr] (flows).
+__global__ void k_pack_solve(DevGrid g, DevBatch b, double base, int pq, int flows, double* out) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= g.nbr) return;
     const size_t B = (size_t)b.B;
+    if (k < g.n) {
+        const double vmi = b.vm[k * B], vai = b.va[k * B];
+        out[k] = vmi;
+        out[g.n + k] = vai * 180.0 / 3.14159265358979323846;
+        if (pq) {
+            double pi = 0.0, qi = 0.0;
+            for (int p = g.yRowPtr[k]; p < g.yRowPtr[k + 1]; p++) {
+                const int j = g.yCol[p];
+                const double G = g.yG[p], Bv = g.yB[p], vmj = b.vm[j * B];
+                double sn, cs;
+                sincos(vai - b.va[j * B], &sn, &cs);
+                pi += vmj * (G * cs + Bv * sn);
+                qi += vmj * (G * sn - Bv * cs);
+            }
+            out[2 * g.n + k] = vmi * pi * base;
+            out[3 * g.n + k] = vmi * qi * base;
+        }
+    }
+    if (!flows) return;
+    double* loading = out + 4 * (size_t)g.n;
+    double* sfo = loading + g.nbr;
+    double* sto = sfo + 2 * (size_t)g.nbr;
+    if (k >= g.nbr) return;
     if (!g.brOn[k]) {
         loading[k] = 0; sfo[2 * k] = sfo[2 * k + 1] = sto[2 * k] = sto[2 * k + 1] = 0;
         return;
@@ -1702,7 +1764,9 @@ struct Workspace {
     DevBuf vm, va, lu, piv, y, z, rhs64, refine, maxMis, maxDx, startMis, finalMis, status, iters, convIters, active, flags, outage,
         loadScale, activeCount;
     DevBuf code, value, maxLoad, minVmNeg, maxVmB, worstBnd, chunkCount, chunkOffset, outKind, outElem, outVal, pq;
-    DevBuf startVm, startVa;
+    DevBuf startVm, startVa, baseOut;
+    DevBuf stage;                // a call's load scales or states, a system a row
+    DevBuf limLo, limHi, busId;  // a screen's voltage limits and bus ids
 };
 
 // The partial-pivoting re-solve of one grid (or matrix pattern): the matrix's cells by column (Symbolic::aColPtr,
@@ -1776,6 +1840,8 @@ struct gs_grid {
     int split = 0;      // first level run by the persistent kernels (factorisation)
     int splitB = 0;     // first level run by the persistent kernels in the triangular solves
     gs::DevSolo solo{};  // one block's shared-memory program of the grid, where its factors fit (on)
+    gs::DevShared shared{};  // a cluster's program, where the factors fit one but not a block (on)
+    gs::DevBuf sharedScratch; // its exports and upper solutions (calls on the context's stream)
     gs::DevBuf soloNext; // its system counter and step maximum (calls on the context's stream)
     int tailSplit = 0;  // first level the few-systems path runs as one CTA per system
     int tailMax = gs::kTailMaxSystems;  // the few-systems path takes over at this many systems still stepping
@@ -1900,6 +1966,47 @@ int SubtreeCutFor(const gs_grid* G, double bytes) {
         best = cut;
     }
     return best;
+}
+
+int UploadShared(gs_grid* G, const SharedProgram& S) {
+    gs_ctx* ctx = G->ctx;
+    DevShared& d = G->shared;
+    std::vector<int> ints;
+    auto put = [&](const std::vector<int32_t>& v) {
+        const int at = (int)ints.size();
+        ints.insert(ints.end(), v.begin(), v.end());
+        return at;
+    };
+    std::vector<DevSharedBlock> blocks;
+    size_t chunks = 0;
+    for (const SharedBlock& b : S.blocks) {
+        DevSharedBlock o{};
+        o.nVal = b.nVal; o.nDinv = b.nDinv; o.nLu = (int)b.from.size(); o.nY = (int)b.yAt.size();
+        o.from = put(b.from); o.yNode = put(b.yNode); o.yAt = put(b.yAt);
+        o.chunks = chunks;
+        chunks += b.chunks.size() / kSoloWords;
+        for (int t = 0; t < S.tiers; t++) {
+            const SharedTier& r = b.tier[t];
+            o.tier[t] = {put(r.down), put(r.up), (int)r.importAt.size(), put(r.importAt), put(r.importPtr), put(r.importIdx),
+                         (int)r.ghostAt.size(), put(r.ghostUp), put(r.ghostAt), (int)r.ownAt.size(), put(r.ownUp), put(r.ownAt)};
+        }
+        blocks.push_back(o);
+    }
+    int rc;
+    if ((rc = Upload(G, blocks, &d.blocks)) != GS_OK || (rc = Upload(G, ints, &d.ints)) != GS_OK) return rc;
+    auto buf = std::make_unique<DevBuf>();
+    GS_CUDA(buf->alloc(chunks * kSoloWords * 4));
+    size_t at = 0;
+    for (const SharedBlock& b : S.blocks) {
+        GS_CUDA(cudaMemcpy(buf->as<char>() + at, b.chunks.data(), b.chunks.size() * 4, cudaMemcpyHostToDevice));
+        at += b.chunks.size() * 4;
+    }
+    d.chunks = buf->as<int4>();
+    G->bufs.push_back(std::move(buf));
+    d.ctas = S.ctas; d.tiers = S.tiers; d.nUpper = S.nUpper; d.nExport = S.nExport;
+    d.smem = S.smem;
+    d.on = 1;
+    return GS_OK;
 }
 
 int UploadGrid(gs_grid* G) {
@@ -2027,6 +2134,12 @@ int UploadGrid(gs_grid* G) {
         d.m = S.m; d.nVal = S.nVal; d.yBase = S.yBase; d.zero = S.zero; d.one = S.one;
         d.on = 1;
     }
+    G->shared.on = 0;
+    if (!G->solo.on && G->ctx->clusterOk && std::getenv("GS_NO_SHARED") == nullptr) {
+        const SharedProgram S = BuildShared(s);
+        if (S.on && (S.ctas <= kClusterCtas || Cluster16Ok()))
+            if ((rc = UploadShared(G, S)) != GS_OK) return rc;
+    }
 #undef UP
     // the few-systems path runs the lowest levels as per-level launches while a phase of them holds more short
     // pieces than one CTA's threads (more than one round of a one-system walk)
@@ -2081,7 +2194,7 @@ int EnsureWs(gs_ctx* ctx, const Symbolic& s, Workspace& w, int B, int precision,
     GS_CUDA(w.flags.alloc(Bz * 4)); GS_CUDA(w.outage.alloc(Bz * 4)); GS_CUDA(w.activeCount.alloc(16));
     GS_CUDA(w.activeList.alloc(Bz * 4));
     GS_CUDA(w.origin.alloc(Bz * 4));
-    GS_CUDA(w.startVm.alloc(s.n * 8)); GS_CUDA(w.startVa.alloc(s.n * 8));
+    GS_CUDA(w.startVm.alloc(s.n * 8)); GS_CUDA(w.startVa.alloc(s.n * 8)); GS_CUDA(w.baseOut.alloc(32));
     if (loadScale) GS_CUDA(w.loadScale.alloc(s.n * Bz * 8));
     if (classifyItems > 0) {
         const int nItems = classifyItems;
@@ -2270,6 +2383,36 @@ int GpStep(gs_grid* G, const DevBatch& cur, const int* dList, int nList, cudaStr
         *launched += 2;
     }
     GS_CUDA(cudaGetLastError());
+    return GS_OK;
+}
+
+// Whether n systems' solves go to the clusters' program rather than the walk over L2. A cluster's blocks are busy with one
+// system alone, so more waves of clusters soon cost more than the walk with its smaller share of blocks a system. Measured
+// (whole solve_batch of 4 to 5 steps, ms, this / the walk): 2,000 buses (4 blocks) 1 system 1.1 / 2.4, 37 2.1 / 5.1,
+// 148 4.6 / 5.1, 296 8.1 / 9.2; 4,000 (8 blocks) 9 2.0 / 7.2, 74 8.1 / 8.5, 148 15.3 / 10.7; one step at 10,000 (16
+// blocks) 6 0.61 / 1.39, 9 1.19 / 2.70, 29 3.2 / 2.0.
+bool SharedTakes(const gs_grid* G, int n) {
+    return G->shared.on && (int64_t)n * G->shared.ctas * G->shared.ctas <= 4096;
+}
+
+// The linear solves of the listed systems of b (FP64) on clusters.
+int SharedSolve(gs_grid* G, const DevBatch& b, const int* list, int n, DevBuf& scratch, cudaStream_t st) {
+    gs_ctx* ctx = G->ctx;
+    const DevShared& P = G->shared;
+    GS_CUDA(scratch.alloc((size_t)n * (P.nExport + P.nUpper) * sizeof(double)));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(n * P.ctas);
+    cfg.blockDim = dim3(kSoloThreads);
+    cfg.dynamicSmemBytes = P.smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = P.ctas;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    GS_CUDA(cudaLaunchKernelEx(&cfg, k_shared, G->view, P, b, list, scratch.as<double>()));
     return GS_OK;
 }
 
@@ -2594,6 +2737,10 @@ int Newton(gs_grid* G, int count, bool useScale, bool startFromWs, const gs_pf_o
                 int gl = 0;
                 if ((rc = GpStep(G, cur, cur.activeList, nActive, st, &gl, true, o.tolerance)) != GS_OK) break;
                 launches += 1 + gl;
+            } else if (SharedTakes(G, nActive)) {
+                if ((rc = SharedSolve(G, cur, cur.activeList, nActive, G->sharedScratch, st)) != GS_OK) break;
+                if (timed) cudaEventRecord(ev[2], st);
+                launches += 2;
             } else {
                 launches += 1 + FewSystemsSolve<double>(g, cur, s, nActive, G->tailSplit, false, st,
                                                         timed ? ev[2] : nullptr, ctx->clusterOk, G->paired);
@@ -3102,14 +3249,17 @@ int SolveBase(gs_grid* G, const gs_pf_opts& o, int* status, int* iters, double* 
     if (rc) return rc;
     rc = RetryStalled(G, 1, &none, nullptr, false, o, ms, nullptr);
     if (rc) return rc;
-    const size_t B = G->ws.B;
     const int n = G->sym.n;
-    // gather system 0 (strided) into the start arrays
-    GS_CUDA(cudaMemcpy2D(G->ws.startVm.p, 8, G->ws.vm.p, B * 8, 8, n, cudaMemcpyDeviceToDevice));
-    GS_CUDA(cudaMemcpy2D(G->ws.startVa.p, 8, G->ws.va.p, B * 8, 8, n, cudaMemcpyDeviceToDevice));
-    GS_CUDA(cudaMemcpy(status, G->ws.status.p, 4, cudaMemcpyDeviceToHost));
-    GS_CUDA(cudaMemcpy(iters, *status == GS_PF_CONVERGED ? G->ws.convIters.p : G->ws.iters.p, 4, cudaMemcpyDeviceToHost));
-    GS_CUDA(cudaMemcpy(mis, G->ws.finalMis.p, 8, cudaMemcpyDeviceToHost));
+    // system 0 (strided) into the start arrays, its control words into one small block
+    k_take_base<<<(n + 127) / 128, 128, 0, ctx->stream>>>(MakeBatch(G, 1, false), n, G->ws.startVm.as<double>(),
+                                                          G->ws.startVa.as<double>(), G->ws.baseOut.as<double>());
+    GS_CUDA(cudaGetLastError());
+    double h[4];
+    GS_CUDA(cudaMemcpyAsync(h, G->ws.baseOut.p, sizeof h, cudaMemcpyDeviceToHost, ctx->stream));
+    GS_CUDA(cudaStreamSynchronize(ctx->stream));
+    *status = (int)h[0];
+    *iters = (int)(*status == GS_PF_CONVERGED ? h[1] : h[2]);
+    *mis = h[3];
     return GS_OK;
 }
 
@@ -3345,52 +3495,25 @@ int gs_pf_solve(gs_grid* G, const gs_pf_opts* opts, gs_pf_result* res) {
     res->iterations = it;
     res->max_mismatch = mis;
     const int n = G->sym.n, nb = G->sym.nbr;
-    const size_t B = G->ws.B;
-    std::vector<double> vm(n), va(n);
-    GS_CUDA(cudaMemcpy(vm.data(), G->ws.startVm.p, n * 8, cudaMemcpyDeviceToHost));
-    GS_CUDA(cudaMemcpy(va.data(), G->ws.startVa.p, n * 8, cudaMemcpyDeviceToHost));
-    for (int i = 0; i < n; i++) {
-        if (res->vm) res->vm[i] = vm[i];
-        if (res->va_deg) res->va_deg[i] = va[i] * 180.0 / 3.14159265358979323846;
-    }
-    if (res->p_inj_mw || res->q_inj_mvar) {
-        GS_CUDA(G->ws.pq.alloc(2 * (size_t)n * B * 8));
-        DevBatch b = MakeBatch(G, 1, false);
-        GS_CUDA(cudaMemset(b.active, 0, B * 4));
-        int one = 1;
-        GS_CUDA(cudaMemcpy(b.active, &one, 4, cudaMemcpyHostToDevice));
-        double* P = G->ws.pq.as<double>();
-        double* Q = P + (size_t)n * B;
-        if (o.precision == GS_PREC_MIXED)
-            k_mismatch_jac<float><<<dim3((n + 7) / 8, B / 32), dim3(32, 8), 0, ctx->stream>>>(G->view, b, 0, P, Q, nullptr, 0);
-        else
-            k_mismatch_jac<double><<<dim3((n + 7) / 8, B / 32), dim3(32, 8), 0, ctx->stream>>>(G->view, b, 0, P, Q, nullptr, 0);
-        GS_CUDA(cudaStreamSynchronize(ctx->stream));
-        std::vector<double> p(n), q(n);
-        GS_CUDA(cudaMemcpy2D(p.data(), 8, P, B * 8, 8, n, cudaMemcpyDeviceToHost));
-        GS_CUDA(cudaMemcpy2D(q.data(), 8, Q, B * 8, 8, n, cudaMemcpyDeviceToHost));
-        for (int i = 0; i < n; i++) {
-            if (res->p_inj_mw) res->p_inj_mw[i] = p[i] * G->host.base;
-            if (res->q_inj_mvar) res->q_inj_mvar[i] = q[i] * G->host.base;
-        }
-    }
-    if (nb > 0 && (res->loading_pct || res->sf_mva || res->st_mva)) {
-        DevBuf tmp;
-        GS_CUDA(tmp.alloc((size_t)nb * 5 * 8));
-        double* ld = tmp.as<double>();
-        double* sf = ld + nb;
-        double* sto = sf + 2 * (size_t)nb;
-        DevBatch b = MakeBatch(G, 1, false);
-        k_lineflows<<<(nb + 127) / 128, 128, 0, ctx->stream>>>(G->view, b, G->host.base, ld, sf, sto);
-        GS_CUDA(cudaStreamSynchronize(ctx->stream));
-        std::vector<double> h((size_t)nb * 5);
-        GS_CUDA(cudaMemcpy(h.data(), ld, h.size() * 8, cudaMemcpyDeviceToHost));
-        for (int k = 0; k < nb; k++) {
-            if (res->loading_pct) res->loading_pct[k] = h[k];
-            if (res->sf_mva) { res->sf_mva[2 * k] = h[nb + 2 * k]; res->sf_mva[2 * k + 1] = h[nb + 2 * k + 1]; }
-            if (res->st_mva) { res->st_mva[2 * k] = h[3 * nb + 2 * k]; res->st_mva[2 * k + 1] = h[3 * nb + 2 * k + 1]; }
-        }
-    }
+    // one kernel packs the results, one copy brings them back
+    const bool pq = res->p_inj_mw || res->q_inj_mvar, fl = nb > 0 && (res->loading_pct || res->sf_mva || res->st_mva);
+    const size_t total = 4 * (size_t)n + 5 * (size_t)nb;
+    GS_CUDA(G->ws.pq.alloc(total * 8));
+    double* d = G->ws.pq.as<double>();
+    DevBatch b = MakeBatch(G, 1, false);
+    k_pack_solve<<<(std::max(n, nb) + 127) / 128, 128, 0, ctx->stream>>>(G->view, b, G->host.base, pq ? 1 : 0, fl ? 1 : 0, d);
+    GS_CUDA(cudaGetLastError());
+    std::vector<double> h(total);
+    GS_CUDA(cudaMemcpyAsync(h.data(), d, total * 8, cudaMemcpyDeviceToHost, ctx->stream));
+    GS_CUDA(cudaStreamSynchronize(ctx->stream));
+    auto out = [&](double* dst, size_t at, size_t len) { if (dst && len) std::memcpy(dst, h.data() + at, len * 8); };
+    out(res->vm, 0, n);
+    out(res->va_deg, n, n);
+    out(res->p_inj_mw, 2 * (size_t)n, n);
+    out(res->q_inj_mvar, 3 * (size_t)n, n);
+    out(res->loading_pct, 4 * (size_t)n, nb);
+    out(res->sf_mva, 4 * (size_t)n + nb, 2 * (size_t)nb);
+    out(res->st_mva, 4 * (size_t)n + 3 * (size_t)nb, 2 * (size_t)nb);
     return GS_OK;
 }
 
@@ -3422,11 +3545,12 @@ int gs_pf_solve_batch(gs_grid* G, int32_t count, const double* loadScale, const 
         std::vector<int> out(B, -1);
         for (int k = 0; k < cnt; k++) out[k] = outage ? outage[done + k] : -1;
         GS_CUDA(cudaMemcpy(G->ws.outage.p, out.data(), B * 4, cudaMemcpyHostToDevice));
+        const dim3 tiles((n + 31) / 32, B / 32), blk8(32, 8);
         if (loadScale) {
-            std::vector<double> sc((size_t)n * B, 1.0);
-            for (int k = 0; k < cnt; k++)
-                for (int i = 0; i < n; i++) sc[(size_t)i * B + k] = loadScale[(size_t)(done + k) * n + i];
-            GS_CUDA(cudaMemcpy(G->ws.loadScale.p, sc.data(), sc.size() * 8, cudaMemcpyHostToDevice));
+            GS_CUDA(G->ws.stage.alloc((size_t)cnt * n * 8));
+            GS_CUDA(cudaMemcpyAsync(G->ws.stage.p, loadScale + (size_t)done * n, (size_t)cnt * n * 8, cudaMemcpyHostToDevice, ctx->stream));
+            k_rows_in<<<tiles, blk8, 0, ctx->stream>>>(G->ws.stage.as<double>(), G->ws.loadScale.as<double>(), n, B, cnt);
+            GS_CUDA(cudaGetLastError());
         }
         float ms = 0;
         rc = NewtonDispatch(G, cnt, loadScale != nullptr, false, o, &ms);
@@ -3446,14 +3570,16 @@ int gs_pf_solve_batch(gs_grid* G, int32_t count, const double* loadScale, const 
             if (maxMismatch) maxMismatch[done + k] = mis[k];
         }
         if (vmOut || vaOut) {
-            std::vector<double> v((size_t)n * B);
+            GS_CUDA(G->ws.stage.alloc((size_t)cnt * n * 8));
             for (int pass = 0; pass < 2; pass++) {
                 double* dst = pass == 0 ? vmOut : vaOut;
                 if (!dst) continue;
-                GS_CUDA(cudaMemcpy(v.data(), pass == 0 ? G->ws.vm.p : G->ws.va.p, v.size() * 8, cudaMemcpyDeviceToHost));
-                const double f = pass == 0 ? 1.0 : 180.0 / 3.14159265358979323846;
-                for (int k = 0; k < cnt; k++)
-                    for (int i = 0; i < n; i++) dst[(size_t)(done + k) * n + i] = v[(size_t)i * B + k] * f;
+                k_rows_out<<<tiles, blk8, 0, ctx->stream>>>(pass == 0 ? G->ws.vm.as<double>() : G->ws.va.as<double>(),
+                                                            G->ws.stage.as<double>(), n, B, cnt,
+                                                            pass == 0 ? 1.0 : 180.0 / 3.14159265358979323846);
+                GS_CUDA(cudaGetLastError());
+                GS_CUDA(cudaMemcpyAsync(dst + (size_t)done * n, G->ws.stage.p, (size_t)cnt * n * 8, cudaMemcpyDeviceToHost, ctx->stream));
+                GS_CUDA(cudaStreamSynchronize(ctx->stream));
             }
         }
         done += cnt;
@@ -3667,7 +3793,7 @@ int ScreenOutageLists(gs_grid* G, int nOut, const std::vector<Element>& els, con
             if (!std::isnan(h.vmin[i])) lo[i] = h.vmin[i];
             if (!std::isnan(h.vmax[i])) hi[i] = h.vmax[i];
         }
-    DevBuf dlo, dhi, dbusId;
+    DevBuf &dlo = G->ws.limLo, &dhi = G->ws.limHi, &dbusId = G->ws.busId;
     GS_CUDA(dlo.alloc(n * 8)); GS_CUDA(dhi.alloc(n * 8)); GS_CUDA(dbusId.alloc(n * 4));
     GS_CUDA(cudaMemcpy(dlo.p, lo.data(), n * 8, cudaMemcpyHostToDevice));
     GS_CUDA(cudaMemcpy(dhi.p, hi.data(), n * 8, cudaMemcpyHostToDevice));
@@ -4320,6 +4446,9 @@ cudaError_t SetKernelAttributes() {
     set((const void*)k_newton<double>);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute((const void*)k_solo, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSoloSmemMax);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute((const void*)k_shared, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSoloSmemMax);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute((const void*)k_shared, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     return e;
 }
 }  // namespace gs

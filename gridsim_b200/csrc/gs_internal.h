@@ -216,6 +216,38 @@ struct SoloProgram {
 // The program of s; on = false when its values do not fit a block's shared memory in FP64.
 SoloProgram BuildSolo(const Symbolic& s);
 
+// The same for systems whose factors fit the shared memory of a cluster of `ctas` blocks (gs_shared.cuh). Every node of
+// the elimination tree is in one block and one tier: tier 0 holds the subtrees below a cut, each whole in one block; the
+// last tier the top of the tree, in block 0; where the top is too large for it, a tier between holds the pieces of it that
+// hang below the last tier's part, each in one block. A block runs its `down` stream of a tier (the levels of its nodes
+// there, then its sums towards entries of higher tiers in other blocks: chunks with kSoloExport, whose targets are indices
+// of the exports in global memory); between tiers the cluster meets at a barrier and a block adds the exports to its
+// entries of the next tier (import). Then `up`, the backward substitution, from the last tier down: before a tier a block
+// copies the solution entries of higher tiers that its nodes there read (ghost), after one it leaves its own in global
+// memory.
+constexpr int32_t kSoloExport = 1 << 11;
+struct SharedTier {
+    std::vector<int32_t> down, up;                       // first tables (3 words a warp), chunk indices global
+    std::vector<int32_t> importAt, importPtr, importIdx; // value += the sum of exports importIdx[importPtr[q] .. [q + 1])
+    std::vector<int32_t> ghostUp, ghostAt;               // index among the upper nodes (tiers above 0), value index
+    std::vector<int32_t> ownUp, ownAt;                   // the block's own upper nodes of the tier
+};
+struct SharedBlock {
+    int nVal = 0, nDinv = 0;             // values (zero at nVal - 2, scratch at nVal - 1); reciprocal pivots and a one
+    std::vector<int32_t> from;           // per LU value: the slot its matrix value comes from (-1: fill)
+    std::vector<int32_t> yNode, yAt;     // its right-hand sides: pivot step and value index
+    std::vector<SharedTier> tier;
+    std::vector<int32_t> chunks;
+};
+struct SharedProgram {
+    bool on = false;
+    int ctas = 0, tiers = 0, nUpper = 0, nExport = 0;
+    size_t smem = 0;
+    std::vector<SharedBlock> blocks;
+};
+// The program of s on the smallest cluster (2, 4, 8 or 16 blocks) that holds it; on = false when none does.
+SharedProgram BuildShared(const Symbolic& s);
+
 // Build s.top[which] for values of `elem` bytes within `budget` bytes of shared memory.
 void BuildTopPart(Symbolic& s, int which, size_t elem, size_t budget);
 

@@ -162,7 +162,6 @@ struct DevBatch {
     int B;                  // interleave stride (multiple of 32)
     int count;              // live systems
     int nLevels;            // elimination-tree levels of the grid
-    int own;                // lu and y are one system's own arrays (k_solo), not interleaved; the rest is
     double* vm;             // [n][B]
     double* va;             // [n][B]
     void* lu;               // [nnzLU][B] of the LU type (diagonal slots keep A(k, k))

@@ -51,18 +51,18 @@ __device__ __forceinline__ void cpAsyncWait() { asm volatile("cp.async.wait_grou
 
 extern __shared__ __align__(16) unsigned char soloSmem[];
 
-// This warp's stream: the factorisation with the forward substitution, then the backward substitution. Chunks come
+// This warp's stream of a program (first: its first table). Chunks come
 // through the warp's ring in shared memory three ahead (each lane copies and reads its own words, so the copies need no
 // barrier and no register waits for L2) and into registers before the barrier that ends the level before. After a
 // barrier every operand of a chunk is loaded at once: a level costs the barrier, one shared-memory latency, the products,
 // the halvings of the sum, and on the factorisation's levels the reciprocal.
-__device__ __forceinline__ void soloRun(const DevSolo& P, int ringOff, int* collapsed) {
+__device__ __forceinline__ void soloRun(const int4* chunks, const int* first, int ringOff, int* collapsed, double* exports) {
     constexpr int Q = kSoloRounds, kBytes = kSoloWords * 4;
     constexpr unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int4* src = P.chunks + (size_t)__ldg(P.first + 3 * w) * (kSoloWords / 4) + lane;
-    const int n = __ldg(P.first + 3 * w + 1);
-    const int before = __ldg(P.first + 3 * w + 2);
+    const int4* src = chunks + (size_t)__ldg(first + 3 * w) * (kSoloWords / 4) + lane;
+    const int n = __ldg(first + 3 * w + 1);
+    const int before = __ldg(first + 3 * w + 2);
     // operands straight from the shared array by byte offset: one instruction each
     const int mine = ringOff + w * kSoloSlots * kBytes + lane * 16;
     auto value = [&](int off) { return *reinterpret_cast<const double*>(soloSmem + off); };
@@ -117,7 +117,11 @@ __device__ __forceinline__ void soloRun(const DevSolo& P, int ringOff, int* coll
                 v = diag ? 1.0 / pv : v;
             }
             if (h & kSoloIsBack) v *= dn;
-            *reinterpret_cast<double*>(soloSmem + target) = v;
+            if (h & kSoloExport) {  // base is the zero: the sum itself, negated
+                if (target >= 0) exports[target] = v;
+            } else {
+                *reinterpret_cast<double*>(soloSmem + target) = v;
+            }
         }
         int bars = h >> 12;
         if (bars > 0) barrier();
@@ -150,7 +154,6 @@ __global__ void __launch_bounds__(kSoloThreads, 2) k_solo(DevGrid g, DevSolo P, 
     const int ring = (P.nVal + P.m + 2) / 2 * 16;
     const int tid = threadIdx.x, bd = blockDim.x, n = g.n;
     DevBatch o = b;  // this system's Jacobian and right-hand side are in shared memory
-    o.own = 1;
     o.lu = val;
     o.y = val + P.yBase;
     o.z = nullptr;
@@ -170,7 +173,7 @@ __global__ void __launch_bounds__(kSoloThreads, 2) k_solo(DevGrid g, DevSolo P, 
             __syncthreads();
             double mx = 0.0;
             int bad = 0;
-            for (int q = tid; q < 2 * n; q += bd) busMismatchJac<double, 2>(g, o, q >> 1, s, 1, nullptr, nullptr, mx, bad);
+            for (int q = tid; q < 2 * n; q += bd) busMismatchJac<double, 2, true>(g, o, q >> 1, s, 1, nullptr, nullptr, mx, bad);
             mx = blockMaxD(mx, redD);
             bad = blockOrI(bad, redI);
             if (tid == 0) {
@@ -194,7 +197,7 @@ __global__ void __launch_bounds__(kSoloThreads, 2) k_solo(DevGrid g, DevSolo P, 
             }
             if (sGo == 0) break;
             if (sGo == 2) continue;  // the next pass starts from this state, no step taken
-            if (tid < 32 * kSoloWarps) soloRun(P, ring, &sCollapsed);
+            if (tid < 32 * kSoloWarps) soloRun(P.chunks, P.first, ring, &sCollapsed, nullptr);
             __syncthreads();
             const double* x = val + P.yBase;
             double dx = 0.0;
