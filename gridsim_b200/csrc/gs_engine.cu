@@ -1649,6 +1649,24 @@ __global__ void k_rows_out(const double* __restrict__ in, double* __restrict__ r
     }
 }
 
+// The batched linear solve's solutions (y, pivot order, interleaved) as rows in the order of the unknowns, with the
+// systems' flags: grid (ceil(n / 32), B / 32), block (32, 8).
+__global__ void k_solution_rows(DevBatch b, int n, int cnt, const int* __restrict__ xinv, double* __restrict__ x, int* flags) {
+    __shared__ double t[32][33];
+    const int i0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
+    const double* y = (const double*)b.y;
+    for (int r = threadIdx.y; r < 32; r += 8) {
+        const int i = i0 + r, k = k0 + threadIdx.x;
+        if (i < n && k < cnt) t[r][threadIdx.x] = y[(size_t)xinv[i] * b.B + k];
+    }
+    __syncthreads();
+    for (int r = threadIdx.y; r < 32; r += 8) {
+        const int k = k0 + r, i = i0 + threadIdx.x;
+        if (i < n && k < cnt) x[(size_t)k * n + i] = t[threadIdx.x][r];
+    }
+    if (blockIdx.x == 0 && threadIdx.y == 0 && k0 + (int)threadIdx.x < cnt) flags[k0 + threadIdx.x] = b.flags[k0 + threadIdx.x];
+}
+
 // System 0's state and control words (status, steps when the tolerance was met, steps, mismatch) gathered.
 __global__ void k_take_base(DevBatch b, int n, double* vm, double* va, double* out) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1728,6 +1746,7 @@ struct DevBuf {
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
     ~DevBuf() { if (p) cudaFree(p); }
+    void release() { if (p) cudaFree(p); p = nullptr; bytes = 0; }
     cudaError_t alloc(size_t n) {
         if (p && bytes >= n) return cudaSuccess;
         if (p) { cudaFree(p); p = nullptr; bytes = 0; }
@@ -1805,6 +1824,14 @@ struct StepGraphCache {
 
 }  // namespace gs
 
+// The multi-grid batch's device arrays, kept by the context between calls (allocating and freeing them cost a call of 192
+// cases up to three times its kernel) up to kMultiKeepBytes an array, and given back with it; calls on a context take turns.
+constexpr size_t kMultiKeepBytes = (size_t)1 << 30;
+struct MultiWs {
+    std::mutex mu;
+    gs::DevBuf arena, views, items, sample, next, scale, outage, status, iters, mis, vm, va, steps;
+};
+
 struct MatrixPattern;  // an analysed sparse-matrix pattern of the batched linear solve (kept per context)
 
 struct gs_ctx {
@@ -1816,6 +1843,7 @@ struct gs_ctx {
     int* pinnedCount = nullptr;
     std::map<std::string, int> multiTune;  // the multi-grid batch's CTA shape per set of grids (autotuned)
     std::vector<std::unique_ptr<MatrixPattern>> patterns;  // most recently used last
+    MultiWs multi;
     unsigned long long* noallocScratch = nullptr;  // device address of the allocation-free check's static scratch
     int sms = 148;
     bool clusterOk = false;  // the few-systems cluster walk can be scheduled on this device
@@ -1864,7 +1892,8 @@ struct MatrixPattern {
     int n = 0;
     std::vector<int> rowPtr, colIdx, aSlot;
     std::unique_ptr<gs_grid> grid;  // the pattern's symbolic analysis, schedules and workspace (no Y, no buses)
-    gs::DevBuf dSlot, dPinv;
+    gs::DevBuf dSlot, dPinv, dXinv;        // entries' slots; pivot positions of the right-hand side's rows, of the unknowns
+    gs::DevBuf vals, rhs, x, flags, redo;  // a call's systems, a system a row
 };
 
 gs_ctx::~gs_ctx() = default;
@@ -4117,9 +4146,10 @@ int PatternOf(gs_ctx* ctx, int n, const int* rp, const int* ci, MatrixPattern** 
         for (int i = 0; i < n; i++) pinv[i] = P->grid->sym.pinv[posOfRow[i]];
     }
     GS_CUDA(P->dSlot.alloc(std::max<size_t>(4, P->aSlot.size() * 4)));
-    GS_CUDA(P->dPinv.alloc(pinv.size() * 4));
+    GS_CUDA(P->dPinv.alloc(pinv.size() * 4)); GS_CUDA(P->dXinv.alloc(pinv.size() * 4));
     if (!P->aSlot.empty()) GS_CUDA(cudaMemcpy(P->dSlot.p, P->aSlot.data(), P->aSlot.size() * 4, cudaMemcpyHostToDevice));
     GS_CUDA(cudaMemcpy(P->dPinv.p, pinv.data(), pinv.size() * 4, cudaMemcpyHostToDevice));
+    GS_CUDA(cudaMemcpy(P->dXinv.p, P->grid->sym.pinv.data(), pinv.size() * 4, cudaMemcpyHostToDevice));
     if ((int)v.size() >= kMaxPatterns) v.erase(v.begin());
     v.push_back(std::move(P));
     *out = v.back().get();
@@ -4181,25 +4211,36 @@ int gs_sparse_solve_batch(gs_ctx* ctx, int32_t count, const int32_t* n, const in
     // factorisation fails, else refused for its right-hand side; its x is never written.
     std::map<uint64_t, std::vector<int>> groups;
     std::vector<char> rhsBad(count, 0);
+    uint64_t lastKey = 0;  // the hash of the last well-formed system's pattern
     for (int q = 0; q < count; q++) {
         const int nq = n[q];
         const int* rp = rowPtr + rpOff[q];
         const int* ci = colIdx + nzOff[q];
-        bool ok = rp[0] == 0;
-        for (int i = 0; i < nq && ok; i++) ok = rp[i + 1] >= rp[i];
-        for (int i = 0; i < nq && ok; i++) {
+        // a system with the pattern of the one before it needs no second look at it
+        const bool same = q > 0 && n[q - 1] == nq && (status[q - 1] != GS_LS_MALFORMED) && lastKey != 0 &&
+                          std::equal(rp, rp + nq + 1, rowPtr + rpOff[q - 1]) && std::equal(ci, ci + rp[nq], colIdx + nzOff[q - 1]);
+        bool ok = same || rp[0] == 0;
+        for (int i = 0; i < nq && ok && !same; i++) ok = rp[i + 1] >= rp[i];
+        for (int i = 0; i < nq && ok && !same; i++) {
+            bool rising = true;
+            for (int p = rp[i] + 1; p < rp[i + 1]; p++) rising = rising && ci[p] > ci[p - 1];
+            if (rising) {
+                ok = rp[i] == rp[i + 1] || (ci[rp[i]] >= 0 && ci[rp[i + 1] - 1] < nq);
+                continue;
+            }
             std::vector<int> row(ci + rp[i], ci + rp[i + 1]);
             std::sort(row.begin(), row.end());
             ok = (row.empty() || (row.front() >= 0 && row.back() < nq)) &&
                  std::adjacent_find(row.begin(), row.end()) == row.end();
         }
-        if (!ok) { status[q] = GS_LS_MALFORMED; continue; }
+        if (!ok) { status[q] = GS_LS_MALFORMED; lastKey = 0; continue; }
+        if (!same) lastKey = PatternHash(nq, rp, ci) | 1;  // 0: none
         bool finite = true;
         for (int p = 0; p < rp[nq] && finite; p++) finite = std::isfinite(values[nzOff[q] + p]);
         if (!finite) { status[q] = GS_LS_NON_FINITE_INPUT; continue; }
         for (int i = 0; i < nq && !rhsBad[q]; i++) rhsBad[q] = !std::isfinite(rhs[vOff[q] + i]);
         status[q] = GS_LS_OK;
-        groups[PatternHash(nq, rp, ci)].push_back(q);
+        groups[lastKey].push_back(q);
     }
     gs_pf_opts o;
     gs_pf_opts_default(&o);
@@ -4229,56 +4270,81 @@ int gs_sparse_solve_batch(gs_ctx* ctx, int32_t count, const int32_t* n, const in
                 const int B = ChooseB(G, want, o);
                 if ((rc = EnsureWorkspace(G, B, GS_PREC_FP64, false, false)) != GS_OK) return rc;
                 const int cnt = std::min(B, want);
-                std::vector<double> hv((size_t)cnt * nnz), hb((size_t)cnt * nq);
-                for (int c = 0; c < cnt; c++) {
+                // values and right-hand sides, a system a row: straight from the caller's arrays where they lie so
+                bool inRow = true;
+                for (int c = 0; c < cnt; c++)
+                    inRow = inRow && !rhsBad[same[done + c]] && nzOff[same[done + c]] == nzOff[same[done]] + (int64_t)c * nnz &&
+                            vOff[same[done + c]] == vOff[same[done]] + (int64_t)c * nq;
+                std::vector<double> hv(inRow ? 0 : (size_t)cnt * nnz), hb(inRow ? 0 : (size_t)cnt * nq);
+                for (int c = 0; c < cnt && !inRow; c++) {
                     const int q = same[done + c];
                     std::copy(values + nzOff[q], values + nzOff[q] + nnz, hv.begin() + (size_t)c * nnz);
                     if (rhsBad[q]) std::fill(hb.begin() + (size_t)c * nq, hb.begin() + (size_t)(c + 1) * nq, 0.0);
                     else std::copy(rhs + vOff[q], rhs + vOff[q] + nq, hb.begin() + (size_t)c * nq);
                 }
-                DevBuf dv, db;
-                GS_CUDA(dv.alloc(std::max<size_t>(8, hv.size() * 8)));
-                GS_CUDA(db.alloc(hb.size() * 8));
-                if (!hv.empty()) GS_CUDA(cudaMemcpy(dv.p, hv.data(), hv.size() * 8, cudaMemcpyHostToDevice));
-                GS_CUDA(cudaMemcpy(db.p, hb.data(), hb.size() * 8, cudaMemcpyHostToDevice));
+                DevBuf &dv = P->vals, &db = P->rhs;
+                GS_CUDA(dv.alloc(std::max<size_t>(8, (size_t)cnt * nnz * 8)));
+                GS_CUDA(db.alloc((size_t)cnt * nq * 8));
+                if (nnz > 0)
+                    GS_CUDA(cudaMemcpyAsync(dv.p, inRow ? values + nzOff[same[done]] : hv.data(), (size_t)cnt * nnz * 8,
+                                            cudaMemcpyHostToDevice, ctx->stream));
+                GS_CUDA(cudaMemcpyAsync(db.p, inRow ? rhs + vOff[same[done]] : hb.data(), (size_t)cnt * nq * 8,
+                                        cudaMemcpyHostToDevice, ctx->stream));
                 const DevBatch b = MakeBatch(G, cnt, false);
-                k_load_matrix<<<dim3((std::max(nnz, nq) + 7) / 8, B / 32), dim3(32, 8), 0, ctx->stream>>>(
-                    b, cnt, nnz, nq, P->dSlot.as<int>(), P->dPinv.as<int>(), dv.as<double>(), db.as<double>());
+                auto loadMatrix = [&]() {
+                    k_load_matrix<<<dim3((std::max(nnz, nq) + 7) / 8, B / 32), dim3(32, 8), 0, ctx->stream>>>(
+                        b, cnt, nnz, nq, P->dSlot.as<int>(), P->dPinv.as<int>(), dv.as<double>(), db.as<double>());
+                };
+                GS_CUDA(P->x.alloc((size_t)cnt * nq * 8));
+                GS_CUDA(P->flags.alloc((size_t)cnt * 4));
+                if (G->solo.on) {  // every system in a block's shared memory
+                    const DevSolo& S = G->solo;
+                    k_solo_linear<<<cnt, kSoloThreads, SoloSmem(S.nVal, S.m), ctx->stream>>>(
+                        S, nnz, nq, P->dSlot.as<int>(), P->dPinv.as<int>(), P->dXinv.as<int>(), dv.as<double>(), db.as<double>(),
+                        P->x.as<double>(), P->flags.as<int>());
+                } else {
+                    loadMatrix();
+                    GS_CUDA(cudaGetLastError());
+                    if ((rc = LinearSolve(G, cnt)) != GS_OK) return rc;
+                    k_solution_rows<<<dim3((nq + 31) / 32, B / 32), dim3(32, 8), 0, ctx->stream>>>(
+                        b, nq, cnt, P->dXinv.as<int>(), P->x.as<double>(), P->flags.as<int>());
+                }
                 GS_CUDA(cudaGetLastError());
-                if ((rc = LinearSolve(G, cnt)) != GS_OK) return rc;
-                std::vector<double> y((size_t)nq * B);
+                std::vector<double> y((size_t)cnt * nq);
                 std::vector<int> fl(cnt);
-                GS_CUDA(cudaMemcpyAsync(y.data(), G->ws.y.p, y.size() * 8, cudaMemcpyDeviceToHost, ctx->stream));
-                GS_CUDA(cudaMemcpyAsync(fl.data(), G->ws.flags.p, cnt * 4, cudaMemcpyDeviceToHost, ctx->stream));
+                GS_CUDA(cudaMemcpyAsync(y.data(), P->x.p, y.size() * 8, cudaMemcpyDeviceToHost, ctx->stream));
+                GS_CUDA(cudaMemcpyAsync(fl.data(), P->flags.p, cnt * 4, cudaMemcpyDeviceToHost, ctx->stream));
                 GS_CUDA(cudaStreamSynchronize(ctx->stream));
-                const std::vector<int>& pinv = G->sym.pinv;
                 std::vector<int> redo;  // systems whose static pivot collapsed (or whose solution is not finite)
                 for (int c = 0; c < cnt; c++) {
                     const int q = same[done + c];
+                    const double* xc = y.data() + (size_t)c * nq;
                     bool good = !(fl[c] & kFlagPivotPerturbed);
-                    for (int i = 0; i < nq && good; i++) good = std::isfinite(y[(size_t)pinv[i] * B + c]);
+                    for (int i = 0; i < nq && good; i++) good = std::isfinite(xc[i]);
                     if (!good) { redo.push_back(c); continue; }
                     if (rhsBad[q]) { status[q] = GS_LS_NON_FINITE_INPUT; continue; }
-                    for (int i = 0; i < nq; i++) x[vOff[q] + i] = y[(size_t)pinv[i] * B + c];
+                    std::copy(xc, xc + nq, x + vOff[q]);
                 }
                 if (!redo.empty()) {
                     // solved again with row partial pivoting (the reference's factorisation) from the reloaded
                     // matrix; singular only if that fails too
-                    k_load_matrix<<<dim3((std::max(nnz, nq) + 7) / 8, B / 32), dim3(32, 8), 0, ctx->stream>>>(
-                        b, cnt, nnz, nq, P->dSlot.as<int>(), P->dPinv.as<int>(), dv.as<double>(), db.as<double>());
-                    DevBuf dl;
+                    loadMatrix();
+                    DevBuf& dl = P->redo;
                     GS_CUDA(dl.alloc(redo.size() * 4));
-                    GS_CUDA(cudaMemcpy(dl.p, redo.data(), redo.size() * 4, cudaMemcpyHostToDevice));
+                    GS_CUDA(cudaMemcpyAsync(dl.p, redo.data(), redo.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
                     int gl = 0;
                     if ((rc = GpStep(G, b, dl.as<int>(), (int)redo.size(), ctx->stream, &gl)) != GS_OK) return rc;
-                    GS_CUDA(cudaMemcpyAsync(y.data(), G->ws.y.p, y.size() * 8, cudaMemcpyDeviceToHost, ctx->stream));
-                    GS_CUDA(cudaMemcpyAsync(fl.data(), G->ws.flags.p, cnt * 4, cudaMemcpyDeviceToHost, ctx->stream));
+                    k_solution_rows<<<dim3((nq + 31) / 32, B / 32), dim3(32, 8), 0, ctx->stream>>>(
+                        b, nq, cnt, P->dXinv.as<int>(), P->x.as<double>(), P->flags.as<int>());
+                    GS_CUDA(cudaGetLastError());
+                    GS_CUDA(cudaMemcpyAsync(y.data(), P->x.p, y.size() * 8, cudaMemcpyDeviceToHost, ctx->stream));
+                    GS_CUDA(cudaMemcpyAsync(fl.data(), P->flags.p, cnt * 4, cudaMemcpyDeviceToHost, ctx->stream));
                     GS_CUDA(cudaStreamSynchronize(ctx->stream));
                     for (int c : redo) {
                         const int q = same[done + c];
                         if (fl[c] & kFlagPivotFailed) { status[q] = GS_LS_SINGULAR; continue; }
                         if (rhsBad[q]) { status[q] = GS_LS_NON_FINITE_INPUT; continue; }
-                        for (int i = 0; i < nq; i++) x[vOff[q] + i] = y[(size_t)pinv[i] * B + c];
+                        std::copy(y.begin() + (size_t)c * nq, y.begin() + (size_t)(c + 1) * nq, x + vOff[q]);
                     }
                 }
                 done += cnt;
@@ -4446,6 +4512,8 @@ cudaError_t SetKernelAttributes() {
     set((const void*)k_newton<double>);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute((const void*)k_solo, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSoloSmemMax);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute((const void*)k_solo_linear, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSoloSmemMax);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute((const void*)k_shared, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSoloSmemMax);
     if (e == cudaSuccess) e = cudaFuncSetAttribute((const void*)k_shared, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);

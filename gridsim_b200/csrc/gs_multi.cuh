@@ -298,15 +298,27 @@ extern "C" int gs_pf_solve_multi(gs_ctx* ctx, int32_t nGrids, gs_grid* const* gr
         ctasOf[q] = std::max(1, occ) * sms;
     }
     // the arena holds the largest CTA count that fits in half the free memory
+    MultiWs& ws = ctx->multi;
+    std::lock_guard<std::mutex> turn(ws.mu);
+    struct GiveBack {  // an arena past the bound is not kept
+        MultiWs& w;
+        ~GiveBack() {
+            for (DevBuf* b : {&w.arena, &w.scale, &w.vm, &w.va})
+                if (b->bytes > kMultiKeepBytes) b->release();
+        }
+    } giveBack{ws};
     size_t freeB = 0, totalB = 0;
     GS_CUDA(cudaMemGetInfo(&freeB, &totalB));
+    freeB += ws.arena.bytes;
     const int maxSlots = (int)std::max<size_t>(1, std::min<size_t>((size_t)2048, (freeB / 2) / arena.stride));
     int slots = 1;
     for (int q = 0; q < kCand; q++) {
         ctasOf[q] = std::min(ctasOf[q], maxSlots);
         slots = std::max(slots, ctasOf[q]);
     }
-    DevBuf dArena, dViews, dItems, dSample, dNext, dScale, dOut, dStatus, dIters, dMis, dVm, dVa, dSteps;
+    DevBuf &dArena = ws.arena, &dViews = ws.views, &dItems = ws.items, &dSample = ws.sample, &dNext = ws.next, &dScale = ws.scale,
+           &dOut = ws.outage, &dStatus = ws.status, &dIters = ws.iters, &dMis = ws.mis, &dVm = ws.vm, &dVa = ws.va,
+           &dSteps = ws.steps;
     GS_CUDA(dArena.alloc((size_t)slots * arena.stride));
     arena.base = dArena.as<char>();
     GS_CUDA(dViews.alloc(views.size() * sizeof(DevGrid)));
@@ -328,18 +340,22 @@ extern "C" int gs_pf_solve_multi(gs_ctx* ctx, int32_t nGrids, gs_grid* const* gr
     GS_CUDA(dMis.alloc((size_t)nCases * 8));
     if (vmOut) GS_CUDA(dVm.alloc((size_t)nStates * 8));
     if (vaOut) GS_CUDA(dVa.alloc((size_t)nStates * 8));
+    const double* scaleIn = loadScale ? dScale.as<double>() : nullptr;
+    const int* outIn = outage ? dOut.as<int>() : nullptr;
+    double* vmTo = vmOut ? dVm.as<double>() : nullptr;
+    double* vaTo = vaOut ? dVa.as<double>() : nullptr;
     auto launch = [&](int q, const MultiItem* its, int nIts) {
         const size_t sm = (candTop[q] ? topBytes : 0) + queueBytes;
         const int qOff = candTop[q] ? (int)topBytes : 0;
         if (mixed)
             k_newton<float><<<ctasOf[q], candThreads[q], sm, st>>>(
-                dViews.as<DevGrid>(), its, nIts, dNext.as<int>(), arena, dScale.as<double>(), dOut.as<int>(),
-                dStatus.as<int>(), dIters.as<int>(), dMis.as<double>(), dVm.as<double>(), dVa.as<double>(), o.tolerance,
+                dViews.as<DevGrid>(), its, nIts, dNext.as<int>(), arena, scaleIn, outIn, dStatus.as<int>(),
+                dIters.as<int>(), dMis.as<double>(), vmTo, vaTo, o.tolerance,
                 o.diverge_limit_pu, o.max_iterations, dSteps.as<unsigned long long>(), candTop[q], qOff);
         else
             k_newton<double><<<ctasOf[q], candThreads[q], sm, st>>>(
-                dViews.as<DevGrid>(), its, nIts, dNext.as<int>(), arena, dScale.as<double>(), dOut.as<int>(),
-                dStatus.as<int>(), dIters.as<int>(), dMis.as<double>(), dVm.as<double>(), dVa.as<double>(), o.tolerance,
+                dViews.as<DevGrid>(), its, nIts, dNext.as<int>(), arena, scaleIn, outIn, dStatus.as<int>(),
+                dIters.as<int>(), dMis.as<double>(), vmTo, vaTo, o.tolerance,
                 o.diverge_limit_pu, o.max_iterations, dSteps.as<unsigned long long>(), candTop[q], qOff);
     };
     // autotuner: the CTA shape per set of grids (and precision), from timed trials on a sample of the items

@@ -236,4 +236,26 @@ __global__ void __launch_bounds__(kSoloThreads, 2) k_solo(DevGrid g, DevSolo P, 
     }
 }
 
+// One linear system a block: vals / rhs a system a row, its entries' slots, the pivot positions of the right-hand side's
+// rows and of the unknowns; x a system a row.
+__global__ void __launch_bounds__(kSoloThreads, 2) k_solo_linear(DevSolo P, int nnz, int n, const int* __restrict__ aSlot,
+                                                                 const int* __restrict__ pinv, const int* __restrict__ xinv,
+                                                                 const double* __restrict__ vals, const double* __restrict__ rhs,
+                                                                 double* __restrict__ x, int* flags) {
+    __shared__ int sCollapsed;
+    double* val = reinterpret_cast<double*>(soloSmem);
+    const int tid = threadIdx.x;
+    const size_t s = blockIdx.x;
+    for (int q = tid; q < P.nVal; q += kSoloThreads) val[q] = 0.0;
+    if (tid == 0) { val[P.nVal + P.one] = 1.0; sCollapsed = 0; }
+    __syncthreads();
+    for (int q = tid; q < nnz; q += kSoloThreads) val[aSlot[q]] = vals[s * nnz + q];
+    for (int i = tid; i < n; i += kSoloThreads) val[P.yBase + pinv[i]] = rhs[s * n + i];
+    __syncthreads();
+    if (tid < 32 * kSoloWarps) soloRun(P.chunks, P.first, (P.nVal + P.m + 2) / 2 * 16, &sCollapsed, nullptr);
+    __syncthreads();
+    for (int i = tid; i < n; i += kSoloThreads) x[s * n + i] = val[P.yBase + xinv[i]];
+    if (tid == 0) flags[s] = sCollapsed ? kFlagPivotPerturbed : 0;
+}
+
 }  // namespace gs
