@@ -4550,6 +4550,8 @@ cudaError_t SetKernelAttributes() {
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute((const void*)k_solo, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSoloSmemMax);
     if (e == cudaSuccess)
+        e = cudaFuncSetAttribute((const void*)k_solo_step, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSoloSmemMax);
+    if (e == cudaSuccess)
         e = cudaFuncSetAttribute((const void*)k_solo_linear, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSoloSmemMax);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute((const void*)k_shared, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSoloSmemMax);

@@ -93,6 +93,11 @@ struct Lane {
     double perSlot = 0;  // device bytes of one slot
     int stateSlots = 0;  // states copied out per tick
     bool warm = false;
+    // The linear solves run in shared memory, in FP64 whatever the precision asked for: a block's (the grid's k_solo
+    // program), or a cluster's while all the slots may go there (SharedTakes). The walk over L2 was bound by its barriers: 256
+    // requests on four grids of 100 to 2,000 buses took 12.2 ms, now 5.2.
+    bool onChip = false;
+    DevBuf scratch;      // the clusters' exports, for every slot
     std::unique_ptr<Workspace> ws;
     std::vector<std::unique_ptr<Workspace>> retired;  // batches outgrown, freed when the loop is destroyed
     DevBuf admitD, doneD, stateD, baseVm, baseVa;
@@ -188,7 +193,7 @@ cudaError_t GrowLane(gs_server* S, Lane& L) {
     }
     const Symbolic& s = L.G->sym;
     auto nw = std::make_unique<Workspace>();
-    if (EnsureWs(S->ctx, s, *nw, C2, S->opts.pf.precision, 0, false) != GS_OK) {
+    if (EnsureWs(S->ctx, s, *nw, C2, L.onChip ? GS_PREC_FP64 : S->opts.pf.precision, 0, false) != GS_OK) {
         std::lock_guard<std::mutex> l(S->mu);
         S->slotBytes -= C2 * L.perSlot;
         cudaGetLastError();
@@ -292,8 +297,15 @@ cudaError_t LaunchB(gs_server* S, Lane& L) {
     if (na > 0) {
         cudaMemsetAsync(b.activeCount, 0, sizeof(int), L.st);
         k_collect_active<<<(L.C + 255) / 256, 256, 0, L.st>>>(b);
-        FewSystemsSolve<T>(g, b, L.G->sym, na, L.G->tailSplit, refine != 0, L.st, nullptr, S->ctx->clusterOk,
-                           L.G->paired);
+        if (L.onChip && L.G->solo.on) {
+            const DevSolo& P = L.G->solo;
+            k_solo_step<<<na, kSoloThreads, SoloSmem(P.nVal, P.m), L.st>>>(g, P, b, b.activeList);
+        } else if (L.onChip) {
+            if (SharedSolve(L.G, b, b.activeList, na, L.scratch, L.st) != GS_OK) return cudaErrorUnknown;
+        } else {
+            FewSystemsSolve<T>(g, b, L.G->sym, na, L.G->tailSplit, refine != 0, L.st, nullptr, S->ctx->clusterOk,
+                               L.G->paired);
+        }
         constexpr int rowsPerBlock = 512;
         k_dxmax<T><<<dim3((m + rowsPerBlock - 1) / rowsPerBlock, (na + 31) / 32), blk8, 0, L.st>>>(g, b, rowsPerBlock, refine,
                                                                                                 b.activeList, na);
@@ -465,7 +477,7 @@ void ServeLoop(gs_server* S, int t, int nt) {
         for (size_t q = 0; q < mine.size() && err == cudaSuccess && rc == GS_OK; q++) {
             const int k = mine[q];
             if (S->batch) progress |= AdvanceBatch(S, *S->lanes[k], k, &rc);
-            else progress |= mixed ? Advance<float>(S, *S->lanes[k], k, &err) : Advance<double>(S, *S->lanes[k], k, &err);
+            else progress |= mixed && !S->lanes[k]->onChip ? Advance<float>(S, *S->lanes[k], k, &err) : Advance<double>(S, *S->lanes[k], k, &err);
         }
         if (err != cudaSuccess || rc != GS_OK) {
             if (err != cudaSuccess) SetErr(S->ctx, GS_ERR_CUDA, std::string("request loop: ") + cudaGetErrorString(err));
@@ -551,11 +563,21 @@ int gs_serve_add_grid(gs_server* S, gs_grid* G, int32_t* index) {
         return GS_OK;
     }
     L->stateSlots = std::min(S->opts.state_slots, S->opts.slots_per_grid);
-    const double per = (double)PerSystemBytes(s, o.precision);
-    const double fixed = (double)L->stateSlots * 2.0 * s.n * 8.0 + 2.0 * s.n * 8.0;
+    double per = (double)PerSystemBytes(s, o.precision);
+    double fixed = (double)L->stateSlots * 2.0 * s.n * 8.0 + 2.0 * s.n * 8.0;
     // every grid starts with 32 slots; it grows by 32 at a time (up to slots_per_grid) while its requests queue and
     // the budget holds the memory (GrowLane)
     const int C = 32;
+    // in shared memory where the budget holds every slot of the lane in FP64
+    const int Cw = S->opts.slots_per_grid;
+    const size_t scratch = G->solo.on ? 0 : (size_t)Cw * (G->shared.nExport + G->shared.nUpper) * sizeof(double);
+    if ((G->solo.on || SharedTakes(G, Cw)) &&
+        S->slotBytes + fixed + (double)scratch + Cw * (double)PerSystemBytes(s, GS_PREC_FP64) <= S->budget) {
+        L->onChip = true;
+        per = (double)PerSystemBytes(s, GS_PREC_FP64);
+        fixed += (double)scratch;
+        if (scratch > 0) GS_CUDA(L->scratch.alloc(scratch));
+    }
     if (S->slotBytes + fixed + C * per > S->budget)
         return SetErr(ctx, GS_ERR_OOM, "the device memory budget of the request loop holds no more slots");
     L->C = C;
@@ -576,7 +598,7 @@ int gs_serve_add_grid(gs_server* S, gs_grid* G, int32_t* index) {
         GS_CUDA(cudaMemcpy(L->baseVa.p, G->ws.startVa.p, (size_t)s.n * 8, cudaMemcpyDeviceToDevice));
     }
     L->ws = std::make_unique<Workspace>();
-    int rc = EnsureWs(ctx, s, *L->ws, C, o.precision, 0, false);
+    int rc = EnsureWs(ctx, s, *L->ws, C, L->onChip ? GS_PREC_FP64 : o.precision, 0, false);
     if (rc) return rc;
     GS_CUDA(cudaMemset(L->ws->active.p, 0, (size_t)C * sizeof(int)));
     // per-slot staging sized for the widest the lane may grow to

@@ -236,6 +236,31 @@ __global__ void __launch_bounds__(kSoloThreads, 2) k_solo(DevGrid g, DevSolo P, 
     }
 }
 
+// The linear solves of the listed systems of batch b (FP64, batch-interleaved), a block each: the Jacobian's values in lu
+// (read only), the right-hand side in y, which becomes the solution. Steps of the request loop, whose systems join and
+// leave between steps: the block's memory is refilled for each.
+__global__ void __launch_bounds__(kSoloThreads, 2) k_solo_step(DevGrid g, DevSolo P, DevBatch b, const int* list) {
+    __shared__ int sCollapsed;
+    double* val = reinterpret_cast<double*>(soloSmem);
+    const int tid = threadIdx.x, s = list[blockIdx.x];
+    const size_t B = (size_t)b.B;
+    const double* lu = (const double*)b.lu + s;
+    double* y = (double*)b.y + s;
+    for (int q = tid; q < P.nVal; q += kSoloThreads) val[q] = 0.0;
+    if (tid == 0) { val[P.nVal + P.one] = 1.0; sCollapsed = 0; }
+    __syncthreads();
+    for (int p = tid; p < 4 * g.yRowPtr[g.n]; p += kSoloThreads) {
+        const int at = g.ySlot[p];
+        if (at >= 0) val[at] = lu[at * B];
+    }
+    for (int k = tid; k < P.m; k += kSoloThreads) val[P.yBase + k] = y[k * B];
+    __syncthreads();
+    if (tid < 32 * kSoloWarps) soloRun(P.chunks, P.first, (P.nVal + P.m + 2) / 2 * 16, &sCollapsed, nullptr);
+    __syncthreads();
+    for (int k = tid; k < P.m; k += kSoloThreads) y[k * B] = val[P.yBase + k];
+    if (tid == 0 && sCollapsed) atomicOr(&b.flags[s], kFlagPivotPerturbed);
+}
+
 // One linear system a block: vals / rhs a system a row, its entries' slots, the pivot positions of the right-hand side's
 // rows and of the unknowns; x a system a row.
 __global__ void __launch_bounds__(kSoloThreads, 2) k_solo_linear(DevSolo P, int nnz, int n, const int* __restrict__ aSlot,

@@ -8,6 +8,7 @@ import pytest
 import oracle
 from gridsim_b200 import _abi, synthetic
 from gridsim_b200.engine import ContingencyAnalysis, PowerFlowOptions, SparseNewtonRaphsonPowerFlow, study_options
+from gridsim_b200.serving import LoadFlowServer, drain
 
 pytestmark = pytest.mark.gpu
 
@@ -63,3 +64,30 @@ def test_cluster_solves_match_the_oracle(n_bus, count):
         assert got["status"][k] == ref["status"] and got["iterations"][k] == ref["iterations"]
         assert np.abs(got["vm"][k] - ref["vm"]).max() <= 1e-8
         assert np.radians(np.abs(got["va_deg"][k] - ref["va_deg"])).max() <= 1e-8
+
+
+# the request loop's steps: a block's program (k_solo_step) at its smallest, an odd size and near its largest, a cluster's of
+# two and four blocks, and the first size whose lanes stay on the walk (eight blocks and 128 slots)
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("n_bus", [6, 31, 640, 1000, 2000, 4000])
+def test_request_steps_match_the_oracle(n_bus, precision):
+    m = synthetic.make_grid(n_bus, n_bus + n_bus // 3 + 1, max(1, n_bus // 8), seed=3)
+    ok = np.nonzero(~synthetic.bridges(m) & (m.br_in_service != 0))[0][:40]
+    opt = PowerFlowOptions(precision=precision, max_iterations=20, warm_start_from_base=True)
+    ref = oracle.screen(m, ok, PowerFlowOptions(max_iterations=20, warm_start_from_base=True).to_c(), keep_states=True)
+    srv = LoadFlowServer(opt, slots_per_grid=128)
+    srv.add_grid(m)
+    srv.start()
+    try:
+        tickets = srv.submit([(0, int(k), 1) for k in ok])
+        got = {r.ticket: r for r in drain(srv, len(ok))}
+    finally:
+        srv.close()
+    vm, va = np.asarray(ref["vm"]).reshape(len(ok), -1), np.asarray(ref["va_deg"]).reshape(len(ok), -1)
+    for k, t in enumerate(tickets):
+        r = got[int(t)]
+        assert r.status == ref["status"][k]
+        if ref["status"][k] == _abi.PF_CONVERGED:
+            assert r.iterations == ref["iterations"][k]
+            assert np.abs(r.vm - vm[k]).max() <= 1e-8
+            assert np.radians(np.abs(r.va_deg - va[k])).max() <= 1e-8
