@@ -18,6 +18,8 @@
 //                        (NewtonShell.ApplyStep :128-136, MaxUndampedStep 0.4, VmFloorPu 0.01).
 // Steps 3-5 are captured once per batch into a CUDA graph and replayed every iteration; the host reads
 // one counter (systems still active) per iteration.
+// Grids whose factors fit a block's shared memory run the whole iteration in one launch instead (k_solo), and the last
+// few systems of larger grids solve in a cluster's (k_shared).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -27,6 +29,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <future>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -2085,6 +2088,17 @@ int UploadGrid(gs_grid* G) {
     const HostGrid& h = G->host;
     const Symbolic& s = G->sym;
     DevGrid& v = G->view;
+    // the shared-memory programs are built while the rest is uploaded (a thread where one is to be had); a bare matrix
+    // pattern has no use for a cluster's
+    struct Programs { SoloProgram solo; SharedProgram shared; };
+    const bool wantSolo = std::getenv("GS_NO_SOLO") == nullptr;
+    const bool wantShared = G->ctx->clusterOk && h.n > 0 && std::getenv("GS_NO_SHARED") == nullptr;
+    std::future<Programs> building = std::async(std::launch::async | std::launch::deferred, [&s, wantSolo, wantShared]() {
+        Programs p;
+        if (wantSolo) p.solo = BuildSolo(s);
+        if (!p.solo.on && wantShared) p.shared = BuildShared(s);
+        return p;
+    });
     v.n = s.n; v.m = s.m; v.nnzY = s.nnzY; v.nbr = s.nbr; v.nnzLU = s.nnzLU; v.nLevels = s.nLevels;
     v.qlim = s.qlim ? 1 : 0;
     v.qlimOn = v.qlim;
@@ -2198,7 +2212,8 @@ int UploadGrid(gs_grid* G) {
         v.psLevels = P.nLevels;
     }
     G->solo.on = 0;
-    if (const SoloProgram S = BuildSolo(s); S.on && std::getenv("GS_NO_SOLO") == nullptr) {
+    const Programs built = building.get();
+    if (const SoloProgram& S = built.solo; S.on) {
         DevSolo& d = G->solo;
         std::vector<int4> chunks(S.chunks.size() / 4);
         std::memcpy(chunks.data(), S.chunks.data(), S.chunks.size() * 4);
@@ -2207,8 +2222,8 @@ int UploadGrid(gs_grid* G) {
         d.on = 1;
     }
     G->shared.on = 0;
-    if (!G->solo.on && G->ctx->clusterOk && std::getenv("GS_NO_SHARED") == nullptr) {
-        const SharedProgram S = BuildShared(s);
+    {
+        const SharedProgram& S = built.shared;
         if (S.on && (S.ctas <= kClusterCtas || Cluster16Ok()))
             if ((rc = UploadShared(G, S)) != GS_OK) return rc;
     }

@@ -2,6 +2,7 @@
 // the entries of every elimination level cut into warp-sized bundles and dealt to the warps.
 #include <algorithm>
 #include <atomic>
+#include <future>
 #include <thread>
 
 #include "gs_internal.h"
@@ -392,11 +393,13 @@ bool BuildSharedOn(const Symbolic& s, int C, double part, SharedProgram& P) {
             Emit(u, B.chunks, B.tier[t].up);
         }
     };
-    std::vector<std::thread> threads;
     std::atomic<int> next{0};
-    for (int w = 0; w < std::min(C, std::max(1, (int)std::thread::hardware_concurrency())); w++)
-        threads.emplace_back([&]() { for (int q; (q = next++) < C;) build(q); });
-    for (auto& t : threads) t.join();
+    auto work = [&]() { for (int q; (q = next++) < C;) build(q); };
+    std::vector<std::future<void>> threads;
+    for (int w = 1; w < std::min(C, std::max(1, (int)std::thread::hardware_concurrency())); w++)
+        threads.push_back(std::async(std::launch::async | std::launch::deferred, work));  // deferred: no thread to be had
+    work();
+    for (auto& t : threads) t.get();
     P.on = true;
     return true;
 }
