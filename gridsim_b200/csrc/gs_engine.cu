@@ -2091,11 +2091,10 @@ int UploadGrid(gs_grid* G) {
     // the shared-memory programs are built while the rest is uploaded (a thread where one is to be had); a bare matrix
     // pattern has no use for a cluster's
     struct Programs { SoloProgram solo; SharedProgram shared; };
-    const bool wantSolo = std::getenv("GS_NO_SOLO") == nullptr;
-    const bool wantShared = G->ctx->clusterOk && h.n > 0 && std::getenv("GS_NO_SHARED") == nullptr;
-    std::future<Programs> building = std::async(std::launch::async | std::launch::deferred, [&s, wantSolo, wantShared]() {
+    const bool wantShared = G->ctx->clusterOk && h.n > 0;
+    std::future<Programs> building = std::async(std::launch::async | std::launch::deferred, [&s, wantShared]() {
         Programs p;
-        if (wantSolo) p.solo = BuildSolo(s);
+        p.solo = BuildSolo(s);
         if (!p.solo.on && wantShared) p.shared = BuildShared(s);
         return p;
     });
