@@ -2057,7 +2057,7 @@ int UploadShared(gs_grid* G, const SharedProgram& S) {
     for (const SharedBlock& b : S.blocks) {
         DevSharedBlock o{};
         o.nVal = b.nVal; o.nDinv = b.nDinv; o.nLu = (int)b.from.size(); o.nY = (int)b.yAt.size();
-        o.from = put(b.from); o.yNode = put(b.yNode); o.yAt = put(b.yAt);
+        o.from = put(b.from); o.yNode = put(b.yNode); o.yAt = put(b.yAt); o.diagAt = put(b.diagAt);
         o.chunks = chunks;
         chunks += b.chunks.size() / kSoloWords;
         for (int t = 0; t < S.tiers; t++) {

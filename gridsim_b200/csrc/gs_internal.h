@@ -224,7 +224,8 @@ SoloProgram BuildSolo(const Symbolic& s);
 // of the exports in global memory); between tiers the cluster meets at a barrier and a block adds the exports to its
 // entries of the next tier (import). Then `up`, the backward substitution, from the last tier down: before a tier a block
 // copies the solution entries of higher tiers that its nodes there read (ghost), after one it leaves its own in global
-// memory.
+// memory. A pivot's floor is relative to the matrix's own diagonal, which an import overwrites: the reciprocal pivots'
+// places hold the matrix's diagonal (diagAt) until the pivot is there.
 constexpr int32_t kSoloExport = 1 << 11;
 struct SharedTier {
     std::vector<int32_t> down, up;                       // first tables (3 words a warp), chunk indices global
@@ -236,6 +237,7 @@ struct SharedBlock {
     int nVal = 0, nDinv = 0;             // values (zero at nVal - 2, scratch at nVal - 1); reciprocal pivots and a one
     std::vector<int32_t> from;           // per LU value: the slot its matrix value comes from (-1: fill)
     std::vector<int32_t> yNode, yAt;     // its right-hand sides: pivot step and value index
+    std::vector<int32_t> diagAt;         // per reciprocal pivot: the value index of its diagonal
     std::vector<SharedTier> tier;
     std::vector<int32_t> chunks;
 };

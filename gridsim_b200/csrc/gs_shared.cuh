@@ -18,7 +18,7 @@ struct DevSharedTier {
 };
 struct DevSharedBlock {
     int nVal, nDinv, nLu, nY;
-    int from, yNode, yAt;
+    int from, yNode, yAt, diagAt;
     size_t chunks;                          // the block's first chunk
     DevSharedTier tier[3];
 };
@@ -52,6 +52,7 @@ __global__ void __launch_bounds__(kSoloThreads, 1) k_shared(DevGrid g, DevShared
     if (tid == 0) { val[nVal + B.nDinv - 1] = 1.0; sCollapsed = 0; }
     __syncthreads();
     for (int k = tid; k < B.nY; k += kSoloThreads) val[__ldg(ints + B.yAt + k)] = y[__ldg(ints + B.yNode + k) * S];
+    for (int k = tid; k < B.nDinv - 1; k += kSoloThreads) val[nVal + k] = val[__ldg(ints + B.diagAt + k)];  // for the pivots' floors
     __syncthreads();
     const int4* chunks = P.chunks + B.chunks * (kSoloWords / 4);
     auto meet = [&]() {
@@ -71,7 +72,7 @@ __global__ void __launch_bounds__(kSoloThreads, 1) k_shared(DevGrid g, DevShared
             }
             __syncthreads();
         }
-        if (tid < 32 * kSoloWarps) soloRun(chunks, ints + R.down, ring, &sCollapsed, ext);
+        if (tid < 32 * kSoloWarps) soloRun<true>(chunks, ints + R.down, ring, &sCollapsed, ext);
     }
     for (int t = P.tiers - 1; t >= 0; t--) {
         const DevSharedTier& R = B.tier[t];
@@ -81,7 +82,7 @@ __global__ void __launch_bounds__(kSoloThreads, 1) k_shared(DevGrid g, DevShared
                 val[__ldg(ints + R.ghostAt + k)] = __ldcg(up + __ldg(ints + R.ghostUp + k));
         }
         __syncthreads();
-        if (tid < 32 * kSoloWarps) soloRun(chunks, ints + R.up, ring, &sCollapsed, ext);
+        if (tid < 32 * kSoloWarps) soloRun<true>(chunks, ints + R.up, ring, &sCollapsed, ext);
         __syncthreads();
         for (int k = tid; k < R.nOwn; k += kSoloThreads) up[__ldg(ints + R.ownUp + k)] = val[__ldg(ints + R.ownAt + k)];
     }

@@ -291,6 +291,7 @@ bool BuildSharedOn(const Symbolic& s, int C, double part, SharedProgram& P) {
             b.from.push_back(hasA[x] ? (int32_t)x : -1);
         }
         dAt[k] = b.nDinv++;
+        b.diagAt.push_back(luAt[s.luBase[k]]);
         if (tier[k] > 0) upIdx[k] = P.nUpper++;
     }
     for (SharedBlock& b : P.blocks) { b.nVal = (int)b.from.size(); b.tier.resize(T); }

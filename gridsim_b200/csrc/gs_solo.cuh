@@ -55,7 +55,10 @@ extern __shared__ __align__(16) unsigned char soloSmem[];
 // through the warp's ring in shared memory three ahead (each lane copies and reads its own words, so the copies need no
 // barrier and no register waits for L2) and into registers before the barrier that ends the level before. After a
 // barrier every operand of a chunk is loaded at once: a level costs the barrier, one shared-memory latency, the products,
-// the halvings of the sum, and on the factorisation's levels the reciprocal.
+// the halvings of the sum, and on the factorisation's levels the reciprocal. A pivot's floor is relative to the matrix's
+// diagonal: the value the sum starts from, or (Imported: that value may hold other blocks' sums too) what is in the
+// reciprocal pivot's place before it.
+template <bool Imported>
 __device__ __forceinline__ void soloRun(const int4* chunks, const int* first, int ringOff, int* collapsed, double* exports) {
     constexpr int Q = kSoloRounds, kBytes = kSoloWords * 4;
     constexpr unsigned full = 0xffffffffu;
@@ -101,7 +104,7 @@ __device__ __forceinline__ void soloRun(const int4* chunks, const int* first, in
         const double base = value(c[0].w), dn = value(c[3].w);
         const int target = c[1].w, h = head;
         const bool diag = (c[2].w & 15) == kSoloDiag;
-        const double mag = fabs(base), fl = diag ? pivotFloor<double>() * (mag > 1.0 ? mag : 1.0) : 0.0;
+        const double mag = fabs(Imported ? dn : base), fl = diag ? pivotFloor<double>() * (mag > 1.0 ? mag : 1.0) : 0.0;
         acc0 += l[0] * (u[0] * d[0]);
         acc1 += l[1] * (u[1] * d[1]);
         acc0 += l[2] * (u[2] * d[2]);
@@ -197,7 +200,7 @@ __global__ void __launch_bounds__(kSoloThreads, 2) k_solo(DevGrid g, DevSolo P, 
             }
             if (sGo == 0) break;
             if (sGo == 2) continue;  // the next pass starts from this state, no step taken
-            if (tid < 32 * kSoloWarps) soloRun(P.chunks, P.first, ring, &sCollapsed, nullptr);
+            if (tid < 32 * kSoloWarps) soloRun<false>(P.chunks, P.first, ring, &sCollapsed, nullptr);
             __syncthreads();
             const double* x = val + P.yBase;
             double dx = 0.0;
@@ -255,7 +258,7 @@ __global__ void __launch_bounds__(kSoloThreads, 2) k_solo_step(DevGrid g, DevSol
     }
     for (int k = tid; k < P.m; k += kSoloThreads) val[P.yBase + k] = y[k * B];
     __syncthreads();
-    if (tid < 32 * kSoloWarps) soloRun(P.chunks, P.first, (P.nVal + P.m + 2) / 2 * 16, &sCollapsed, nullptr);
+    if (tid < 32 * kSoloWarps) soloRun<false>(P.chunks, P.first, (P.nVal + P.m + 2) / 2 * 16, &sCollapsed, nullptr);
     __syncthreads();
     for (int k = tid; k < P.m; k += kSoloThreads) y[k * B] = val[P.yBase + k];
     if (tid == 0 && sCollapsed) atomicOr(&b.flags[s], kFlagPivotPerturbed);
@@ -277,7 +280,7 @@ __global__ void __launch_bounds__(kSoloThreads, 2) k_solo_linear(DevSolo P, int 
     for (int q = tid; q < nnz; q += kSoloThreads) val[aSlot[q]] = vals[s * nnz + q];
     for (int i = tid; i < n; i += kSoloThreads) val[P.yBase + pinv[i]] = rhs[s * n + i];
     __syncthreads();
-    if (tid < 32 * kSoloWarps) soloRun(P.chunks, P.first, (P.nVal + P.m + 2) / 2 * 16, &sCollapsed, nullptr);
+    if (tid < 32 * kSoloWarps) soloRun<false>(P.chunks, P.first, (P.nVal + P.m + 2) / 2 * 16, &sCollapsed, nullptr);
     __syncthreads();
     for (int i = tid; i < n; i += kSoloThreads) x[s * n + i] = val[P.yBase + xinv[i]];
     if (tid == 0) flags[s] = sCollapsed ? kFlagPivotPerturbed : 0;
