@@ -95,8 +95,8 @@ struct Lane {
     bool warm = false;
     // The linear solves run in shared memory, in FP64 whatever the precision asked for: a block's (the grid's k_solo
     // program), or a cluster's while all the slots may go there (SharedTakes). The walk over L2 was bound by its barriers: 256
-    // requests on four grids of 100 to 2,000 buses took 12.2 ms, now 5.2.
-    bool onChip = false;
+    // requests on four grids of 100 to 2,000 buses took 12.2 ms, now 5.2. Decided when the loop starts (PlaceLanes).
+    bool onChip = false, placed = false;
     DevBuf scratch;      // the clusters' exports, for every slot
     std::unique_ptr<Workspace> ws;
     std::vector<std::unique_ptr<Workspace>> retired;  // batches outgrown, freed when the loop is destroyed
@@ -316,6 +316,43 @@ cudaError_t LaunchB(gs_server* S, Lane& L) {
     cudaEventRecord(L.evB, L.st);
     L.phase = 2;
     return cudaGetLastError();
+}
+
+// Which lanes solve in shared memory. Their slots are FP64, about twice a mixed lane's FP32 ones, and the clusters need
+// their exports' memory; a lane takes them only where the budget still holds every lane at its full width, outgrown batches
+// included, so that no grid is refused and no lane kept narrower for it. Every grid is known when the loop starts.
+void PlaceLanes(gs_server* S) {
+    auto growth = [](const Lane& L) {  // slots of the batches a lane may still grow into, one after the other
+        double c = 0;
+        for (int w = L.C + 32; w <= L.Cmax; w += 32) c += w;
+        return c;
+    };
+    double need = S->slotBytes;
+    for (auto& L : S->lanes) need += growth(*L) * L->perSlot;
+    for (auto& lp : S->lanes) {
+        Lane& L = *lp;
+        if (L.placed) continue;
+        L.placed = true;
+        if (!L.G->solo.on && !SharedTakes(L.G, L.Cmax)) continue;
+        const Symbolic& s = L.G->sym;
+        const size_t scratch = L.G->solo.on ? 0 : (size_t)L.Cmax * (L.G->shared.nExport + L.G->shared.nUpper) * sizeof(double);
+        const double per = (double)PerSystemBytes(s, GS_PREC_FP64), more = (double)scratch + L.C * (per - L.perSlot);
+        if (need + more + growth(L) * (per - L.perSlot) > S->budget) continue;
+        auto ws = std::make_unique<Workspace>();
+        if (EnsureWs(S->ctx, s, *ws, L.C, GS_PREC_FP64, 0, false) != GS_OK ||
+            (scratch > 0 && L.scratch.alloc(scratch) != cudaSuccess) ||
+            cudaMemset(ws->active.p, 0, (size_t)L.C * sizeof(int)) != cudaSuccess) {
+            cudaGetLastError();  // no memory after all: the lane stays as it is
+            L.scratch.release();
+            continue;
+        }
+        need += more + growth(L) * (per - L.perSlot);
+        S->slotBytes += more;
+        L.perSlot = per;
+        L.onChip = true;
+        L.ws = std::move(ws);
+        L.batch = MakeBatchWs(*L.ws, s.nLevels, L.C, L.C, false);
+    }
 }
 
 // After half B: answer the requests whose states were copied out.
@@ -563,21 +600,11 @@ int gs_serve_add_grid(gs_server* S, gs_grid* G, int32_t* index) {
         return GS_OK;
     }
     L->stateSlots = std::min(S->opts.state_slots, S->opts.slots_per_grid);
-    double per = (double)PerSystemBytes(s, o.precision);
-    double fixed = (double)L->stateSlots * 2.0 * s.n * 8.0 + 2.0 * s.n * 8.0;
+    const double per = (double)PerSystemBytes(s, o.precision);
+    const double fixed = (double)L->stateSlots * 2.0 * s.n * 8.0 + 2.0 * s.n * 8.0;
     // every grid starts with 32 slots; it grows by 32 at a time (up to slots_per_grid) while its requests queue and
     // the budget holds the memory (GrowLane)
     const int C = 32;
-    // in shared memory where the budget holds every slot of the lane in FP64
-    const int Cw = S->opts.slots_per_grid;
-    const size_t scratch = G->solo.on ? 0 : (size_t)Cw * (G->shared.nExport + G->shared.nUpper) * sizeof(double);
-    if ((G->solo.on || SharedTakes(G, Cw)) &&
-        S->slotBytes + fixed + (double)scratch + Cw * (double)PerSystemBytes(s, GS_PREC_FP64) <= S->budget) {
-        L->onChip = true;
-        per = (double)PerSystemBytes(s, GS_PREC_FP64);
-        fixed += (double)scratch;
-        if (scratch > 0) GS_CUDA(L->scratch.alloc(scratch));
-    }
     if (S->slotBytes + fixed + C * per > S->budget)
         return SetErr(ctx, GS_ERR_OOM, "the device memory budget of the request loop holds no more slots");
     L->C = C;
@@ -598,7 +625,7 @@ int gs_serve_add_grid(gs_server* S, gs_grid* G, int32_t* index) {
         GS_CUDA(cudaMemcpy(L->baseVa.p, G->ws.startVa.p, (size_t)s.n * 8, cudaMemcpyDeviceToDevice));
     }
     L->ws = std::make_unique<Workspace>();
-    int rc = EnsureWs(ctx, s, *L->ws, C, L->onChip ? GS_PREC_FP64 : o.precision, 0, false);
+    int rc = EnsureWs(ctx, s, *L->ws, C, o.precision, 0, false);
     if (rc) return rc;
     GS_CUDA(cudaMemset(L->ws->active.p, 0, (size_t)C * sizeof(int)));
     // per-slot staging sized for the widest the lane may grow to
@@ -630,13 +657,19 @@ int gs_serve_start(gs_server* S) {
     using namespace gs;
     using namespace gs::serve;
     if (!S) return GS_ERR_INVALID_ARG;
-    if (S->started) return SetErr(S->ctx, GS_ERR_STATE, "the request loop is already running");
-    if (S->lanes.empty()) return SetErr(S->ctx, GS_ERR_STATE, "no grid added");
+    gs_ctx* ctx = S->ctx;
+    if (S->started) return SetErr(ctx, GS_ERR_STATE, "the request loop is already running");
+    if (S->lanes.empty()) return SetErr(ctx, GS_ERR_STATE, "no grid added");
     // scheduler threads: one per grid up to 8 (or as asked); the batch mode runs its solves on the context's one
     // stream, so it keeps one thread
     int nt = S->opts.scheduler_threads > 0 ? S->opts.scheduler_threads : 8;
     nt = std::max(1, std::min<int>(nt, (int)S->lanes.size()));
-    if (S->batch) nt = 1;
+    if (S->batch) {
+        nt = 1;
+    } else {
+        GS_CUDA(cudaSetDevice(ctx->device));
+        PlaceLanes(S);
+    }
     S->inbox.assign(nt, {});
     S->threadsRunning = nt;
     S->started = true;

@@ -431,7 +431,9 @@ typedef struct gs_serve_opts {
                                   requests queue and the budget below holds the memory (admission by device memory) */
     int32_t state_slots;       /* solved states returned per grid and iteration; 0 = 16 */
     double hbm_fraction;       /* share of the free device memory (at gs_serve_create) that all grids' slot batches
-                                  share; 0 = 0.5 */
+                                  share; 0 = 0.5. Booked in the options' precision; gs_serve_start gives a mixed
+                                  loop's grids FP64 slots (solves in shared memory) while every grid at its full
+                                  width still fits */
     int32_t scheduler_threads; /* host threads that launch the grids' iterations (each owns every k-th grid); 0 = one
                                   per grid up to 8; the batch mode (Q limits, the DC retry, partial pivoting) uses one */
     int32_t reserved[7];
