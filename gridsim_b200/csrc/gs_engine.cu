@@ -2472,6 +2472,20 @@ int GpStep(gs_grid* G, const DevBatch& cur, const int* dList, int nList, cudaStr
     return GS_OK;
 }
 
+// Whether a Newton run of `count` systems goes to k_solo, where the grid has a block's program. A block takes one system
+// whatever its size, so small systems in large batches are cheaper level by level, all systems side by side in L2. Measured
+// (whole solve_batch of 3 to 4 steps, FP64, ms, k_solo / level by level): 5 buses 1,000 systems 0.33 / 0.37, 4,000 0.56 /
+// 0.41; 30 buses 2,000 0.55 / 0.84, 4,000 0.92 / 0.88, 20,000 3.5 / 2.1; 57 buses 2,000 0.82 / 0.97, 20,000 5.9 / 4.2,
+// 100,000 (past L2) 27.7 / 30.3; 80 buses 20,000 7.6 / 6.3, 100,000 38 / 48; 120 buses (2,142 LU values) 4,000 2.0 / 2.3,
+// 20,000 8.5 / 10.2. The level kernels refine mixed steps, so the lines of mixed precision lie higher: 30 buses 4,000 0.90 /
+// 1.10, 8,000 1.57 / 1.36.
+bool SoloTakes(const gs_grid* G, int count, bool mixed) {
+    if (!G->solo.on) return false;
+    const Symbolic& s = G->sym;
+    if (count <= (mixed ? std::min(6000, 1800 + 90 * s.m) : std::min(4000, 1800 + 40 * s.m))) return true;
+    return s.nnzLU >= 2000 || (s.nnzLU >= 800 && (double)count * (double)s.nnzLU * 8.0 >= 512e6);
+}
+
 // Whether n systems' solves go to the clusters' program rather than the walk over L2. A cluster's blocks are busy with one
 // system alone, so more waves of clusters soon cost more than the walk with its smaller share of blocks a system. Measured
 // (whole solve_batch of 4 to 5 steps, ms, this / the walk): 2,000 buses (4 blocks) 1 system 1.1 / 2.4, 37 2.1 / 5.1,
@@ -2530,7 +2544,7 @@ int Newton(gs_grid* G, int count, bool useScale, bool startFromWs, const gs_pf_o
     GS_CUDA(cudaGetLastError());
     // with Q limits every pass may take up to max_iterations steps (plus the step-less pass switches)
     const int maxLoop = g.qlim ? (o.max_iterations + 2) * (g.qlimMaxPasses + 2) : o.max_iterations + 4;
-    if (G->solo.on && !G->gpMode && o.phase_timing == 0) {
+    if (SoloTakes(G, count, sizeof(T) < sizeof(double)) && !G->gpMode && o.phase_timing == 0) {
         // the factors fit a block's shared memory: every system's whole run in one launch
         const DevSolo& P = G->solo;
         const size_t smem = SoloSmem(P.nVal, P.m);
