@@ -2043,6 +2043,31 @@ int SubtreeCutFor(const gs_grid* G, double bytes) {
     return best;
 }
 
+void SharedConfig(int clusters, int ctas, size_t smem, cudaLaunchAttribute* attr, cudaLaunchConfig_t* cfg) {
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = ctas;
+    attr->val.clusterDim.y = 1;
+    attr->val.clusterDim.z = 1;
+    *cfg = cudaLaunchConfig_t{};
+    cfg->gridDim = dim3(clusters * ctas);
+    cfg->blockDim = dim3(kSoloThreads);
+    cfg->dynamicSmemBytes = smem;
+    cfg->attrs = attr;
+    cfg->numAttrs = 1;
+}
+
+// The clusters of k_shared that can be resident at once with this many blocks and this much memory a block. (The walk's
+// clusters have 64 KB a block: that they fit says nothing of these, a whole SM's memory a block.)
+int SharedClusters(int ctas, size_t smem) {
+    cudaLaunchAttribute attr;
+    cudaLaunchConfig_t cfg;
+    SharedConfig(1, ctas, smem, &attr, &cfg);
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k_shared, &cfg) == cudaSuccess) return n;
+    cudaGetLastError();
+    return 0;
+}
+
 int UploadShared(gs_grid* G, const SharedProgram& S) {
     gs_ctx* ctx = G->ctx;
     DevShared& d = G->shared;
@@ -2222,9 +2247,8 @@ int UploadGrid(gs_grid* G) {
     }
     G->shared.on = 0;
     {
-        const SharedProgram& S = built.shared;
-        if (S.on && (S.ctas <= kClusterCtas || Cluster16Ok()))
-            if ((rc = UploadShared(G, S)) != GS_OK) return rc;
+        const SharedProgram& S = built.shared;  // without it the walks over L2 take the few-systems steps
+        if (SharedRuns(S, SharedClusters) && (rc = UploadShared(G, S)) != GS_OK) return rc;
     }
 #undef UP
     // the few-systems path runs the lowest levels as per-level launches while a phase of them holds more short
@@ -2496,24 +2520,14 @@ bool SharedTakes(const gs_grid* G, int n) {
 }
 
 // The linear solves of the listed systems of b (FP64) on clusters.
-int SharedSolve(gs_grid* G, const DevBatch& b, const int* list, int n, DevBuf& scratch, cudaStream_t st) {
-    gs_ctx* ctx = G->ctx;
+cudaError_t SharedSolve(gs_grid* G, const DevBatch& b, const int* list, int n, DevBuf& scratch, cudaStream_t st) {
     const DevShared& P = G->shared;
-    GS_CUDA(scratch.alloc((size_t)n * (P.nExport + P.nUpper) * sizeof(double)));
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(n * P.ctas);
-    cfg.blockDim = dim3(kSoloThreads);
-    cfg.dynamicSmemBytes = P.smem;
+    if (cudaError_t e = scratch.alloc((size_t)n * (P.nExport + P.nUpper) * sizeof(double)); e != cudaSuccess) return e;
+    cudaLaunchAttribute attr;
+    cudaLaunchConfig_t cfg;
+    SharedConfig(n, P.ctas, P.smem, &attr, &cfg);
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = P.ctas;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    GS_CUDA(cudaLaunchKernelEx(&cfg, k_shared, G->view, P, b, list, scratch.as<double>()));
-    return GS_OK;
+    return cudaLaunchKernelEx(&cfg, k_shared, G->view, P, b, list, scratch.as<double>());
 }
 
 struct NewtonStats {
@@ -2838,7 +2852,10 @@ int Newton(gs_grid* G, int count, bool useScale, bool startFromWs, const gs_pf_o
                 if ((rc = GpStep(G, cur, cur.activeList, nActive, st, &gl, true, o.tolerance)) != GS_OK) break;
                 launches += 1 + gl;
             } else if (SharedTakes(G, nActive)) {
-                if ((rc = SharedSolve(G, cur, cur.activeList, nActive, G->sharedScratch, st)) != GS_OK) break;
+                if (cudaError_t e = SharedSolve(G, cur, cur.activeList, nActive, G->sharedScratch, st); e != cudaSuccess) {
+                    rc = SetErr(ctx, GS_ERR_CUDA, std::string("cluster solve: ") + cudaGetErrorString(e));
+                    break;
+                }
                 if (timed) cudaEventRecord(ev[2], st);
                 launches += 2;
             } else {

@@ -249,6 +249,11 @@ struct SharedProgram {
 };
 // The program of s on the smallest cluster (2, 4, 8 or 16 blocks) that holds it; on = false when none does.
 SharedProgram BuildShared(const Symbolic& s);
+// Whether the device may run P: clusters(ctas, smem) is how many of its clusters can be resident at once.
+template <typename Clusters>
+bool SharedRuns(const SharedProgram& P, Clusters clusters) {
+    return P.on && clusters(P.ctas, P.smem) >= 1;
+}
 
 // Build s.top[which] for values of `elem` bytes within `budget` bytes of shared memory.
 void BuildTopPart(Symbolic& s, int which, size_t elem, size_t budget);

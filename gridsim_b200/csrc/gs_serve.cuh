@@ -301,7 +301,7 @@ cudaError_t LaunchB(gs_server* S, Lane& L) {
             const DevSolo& P = L.G->solo;
             k_solo_step<<<na, kSoloThreads, SoloSmem(P.nVal, P.m), L.st>>>(g, P, b, b.activeList);
         } else if (L.onChip) {
-            if (SharedSolve(L.G, b, b.activeList, na, L.scratch, L.st) != GS_OK) return cudaErrorUnknown;
+            if (cudaError_t e = SharedSolve(L.G, b, b.activeList, na, L.scratch, L.st); e != cudaSuccess) return e;
         } else {
             FewSystemsSolve<T>(g, b, L.G->sym, na, L.G->tailSplit, refine != 0, L.st, nullptr, S->ctx->clusterOk,
                                L.G->paired);
