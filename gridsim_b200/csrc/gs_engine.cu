@@ -1870,9 +1870,19 @@ struct StepGraphCache {
 
 }  // namespace gs
 
+// What a call leaves allocated for the next one beside the workspaces: arrays of up to kKeepBytes. KeepBounded gives the
+// larger ones of the listed arrays back when the call ends (freeing waits for the kernels that use them).
+constexpr size_t kKeepBytes = (size_t)1 << 30;
+struct KeepBounded {
+    std::vector<gs::DevBuf*> bufs;
+    ~KeepBounded() {
+        for (gs::DevBuf* b : bufs)
+            if (b->bytes > kKeepBytes) b->release();
+    }
+};
+
 // The multi-grid batch's device arrays, kept by the context between calls (allocating and freeing them cost a call of 192
-// cases up to three times its kernel) up to kMultiKeepBytes an array, and given back with it; calls on a context take turns.
-constexpr size_t kMultiKeepBytes = (size_t)1 << 30;
+// cases up to three times its kernel) and given back with it; calls on a context take turns.
 struct MultiWs {
     std::mutex mu;
     gs::DevBuf arena, views, items, sample, next, scale, outage, status, iters, mis, vm, va, steps;
@@ -3653,6 +3663,7 @@ int gs_pf_solve_batch(gs_grid* G, int32_t count, const double* loadScale, const 
                 return SetErr(ctx, GS_ERR_INVALID_ARG, "outage index out of range or out of service");
     GS_CUDA(cudaSetDevice(ctx->device));
     const int n = s.n;
+    KeepBounded keep{{&G->ws.stage}};
     int done = 0;
     while (done < count) {
         int B = ChooseB(G, count - done, o);
@@ -4346,6 +4357,7 @@ int gs_sparse_solve_batch(gs_ctx* ctx, int32_t count, const int32_t* n, const in
             int rc = PatternOf(ctx, nq, rp0, ci0, &P);
             if (rc) return rc;
             gs_grid* G = P->grid.get();
+            KeepBounded keep{{&P->vals, &P->rhs, &P->x}};
             int done = 0;
             while (done < (int)same.size()) {
                 const int want = (int)same.size() - done;

@@ -300,13 +300,7 @@ extern "C" int gs_pf_solve_multi(gs_ctx* ctx, int32_t nGrids, gs_grid* const* gr
     // the arena holds the largest CTA count that fits in half the free memory
     MultiWs& ws = ctx->multi;
     std::lock_guard<std::mutex> turn(ws.mu);
-    struct GiveBack {  // an arena past the bound is not kept
-        MultiWs& w;
-        ~GiveBack() {
-            for (DevBuf* b : {&w.arena, &w.scale, &w.vm, &w.va})
-                if (b->bytes > kMultiKeepBytes) b->release();
-        }
-    } giveBack{ws};
+    KeepBounded keep{{&ws.arena, &ws.scale, &ws.vm, &ws.va}};
     size_t freeB = 0, totalB = 0;
     GS_CUDA(cudaMemGetInfo(&freeB, &totalB));
     freeB += ws.arena.bytes;
