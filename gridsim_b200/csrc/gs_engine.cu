@@ -2249,9 +2249,9 @@ int UploadGrid(gs_grid* G) {
     const Programs built = building.get();
     if (const SoloProgram& S = built.solo; S.on) {
         DevSolo& d = G->solo;
-        std::vector<int4> chunks(S.chunks.size() / 4);
-        std::memcpy(chunks.data(), S.chunks.data(), S.chunks.size() * 4);
-        if ((rc = Upload(G, chunks, &d.chunks)) != GS_OK || (rc = Upload(G, S.first, &d.first)) != GS_OK) return rc;
+        const int32_t* chunks = nullptr;
+        if ((rc = Upload(G, S.chunks, &chunks)) != GS_OK || (rc = Upload(G, S.first, &d.first)) != GS_OK) return rc;
+        d.chunks = reinterpret_cast<const int4*>(chunks);
         d.m = S.m; d.nVal = S.nVal; d.yBase = S.yBase; d.zero = S.zero; d.one = S.one;
         d.on = 1;
     }

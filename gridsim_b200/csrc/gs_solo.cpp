@@ -18,13 +18,12 @@ struct Task {
 struct TaskList {
     std::vector<Task> tasks;
     std::vector<SoloPair> pairs;
+    std::vector<int> order;  // the levels' tasks as they are dealt, level after level
     void begin(int out, int kind, int node, int level) {
         tasks.push_back({out, kind, node, level, (int)pairs.size(), (int)pairs.size()});
     }
-    void pair(int a, int c, int j) {
-        pairs.push_back({a, c, j});
-        tasks.back().p1++;
-    }
+    void pair(int a, int c, int j) { pairs.push_back({a, c, j}); }
+    void end() { tasks.back().p1 = (int)pairs.size(); }
     void drop() { tasks.pop_back(); }  // a task without pairs
 };
 
@@ -37,36 +36,51 @@ int Lanes(int pairs, int chunks) {  // the lanes whose share of `pairs` takes at
     return g;
 }
 
-// A warp's chunks so far, and the levels it waits out before the first.
+// The sums order[t0 .. t1) of a list, 2^lg lanes each, as consecutive chunks of one warp; the barriers after them.
+struct Bundle {
+    const TaskList* list;
+    int t0, t1, lg, chunks, head, bars;
+};
+// A warp's bundles so far, and the levels it waits out before the first.
 struct Stream {
-    std::vector<int32_t> chunks;
-    int before = 0;
+    std::vector<Bundle> bundles;
+    int before = 0, chunks = 0;
     bool worked = false;  // in the level before
     void barrier() {
-        if (chunks.empty()) { before++; return; }
-        int32_t* c = chunks.data() + chunks.size() - kSoloWords;
-        for (int lane = 0; lane < 32; lane++) c[(2 * 32 + lane) * 4 + 3] += 1 << 12;
+        if (bundles.empty()) before++;
+        else bundles.back().bars++;
     }
 };
 
-// A level's tasks (all independent) into bundles, dealt to the warps, a barrier after each warp's last one.
-// zero: the zero's value index (the scratch value follows it); pivots: the reciprocal pivots' index, one: a one among them.
+// Where a program's values are. zero: the zero's value index (the scratch value follows it); pivots: the reciprocal pivots'
+// index, one: a one among them.
 struct Place { int zero, pivots, one; };
-void AddLevel(const Place& P, std::vector<Stream>& warps, const SoloPair* pairs, const Task* tasks, int nTasks,
-              bool isExport = false) {
-    const int W = (int)warps.size();
+
+// The tasks of one level (all independent; `order`'s from q0 on) into bundles, dealt to the warps, a barrier after each
+// warp's last one.
+void AddLevel(std::vector<Stream>& warps, TaskList& L, int q0, bool isExport = false) {
+    const int W = (int)warps.size(), q1 = (int)L.order.size();
+    int* order = L.order.data();
+    // longest first
+    thread_local std::vector<int> count, start, sizes, sorted;
     int longest = 0;
-    std::vector<int> count;  // tasks by number of pairs
-    for (int q = 0; q < nTasks; q++) {
-        longest = std::max(longest, tasks[q].size());
-        if ((int)count.size() <= tasks[q].size()) count.resize(tasks[q].size() + 1, 0);
-        count[tasks[q].size()]++;
+    for (int q = q0; q < q1; q++) longest = std::max(longest, L.tasks[order[q]].size());
+    count.assign(longest + 1, 0);
+    for (int q = q0; q < q1; q++) count[L.tasks[order[q]].size()]++;
+    start.resize(longest + 1);
+    sizes.clear();
+    for (int n = longest, at = 0; n >= 0; at += count[n--]) {
+        start[n] = at;
+        if (count[n]) sizes.push_back(n);
     }
+    sorted.resize(q1 - q0);
+    for (int q = q0; q < q1; q++) sorted[start[L.tasks[order[q]].size()]++] = order[q];
+    std::copy(sorted.begin(), sorted.end(), order + q0);
     int best = 1;
     int64_t bestCost = INT64_MAX;
     for (int r : {1, 2, 3, 4, 6, 8, 12, 16}) {
         int64_t lanes = 0;
-        for (int n = 0; n <= longest; n++) lanes += (int64_t)count[n] * Lanes(n, r);
+        for (int n : sizes) lanes += (int64_t)count[n] * Lanes(n, r);
         const int g = Lanes(longest, r);
         int h = 0;
         for (int x = g; x > 1; x /= 2) h++;
@@ -76,78 +90,110 @@ void AddLevel(const Place& P, std::vector<Stream>& warps, const SoloPair* pairs,
         if (c < bestCost) { bestCost = c; best = r; }
         if (r * kSoloRounds >= longest) break;
     }
-    // longest first, the lanes of a sum with it: every power of two a class of its own
-    std::vector<int> order(nTasks);
-    for (int q = 0; q < nTasks; q++) order[q] = q;
-    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return tasks[a].size() > tasks[b].size(); });
-    struct Bundle { int lg, chunks, t0, t1; };
-    std::vector<Bundle> bundles;
-    for (int q = 0; q < nTasks;) {
-        const int g = Lanes(tasks[order[q]].size(), best);
+    // the lanes of a sum with its length: every power of two a class of its own
+    thread_local std::vector<Bundle> bundles;
+    bundles.clear();
+    for (int q = q0; q < q1;) {
+        const int longestHere = L.tasks[order[q]].size(), g = Lanes(longestHere, best);
         int e = 0;
         while ((1 << e) < g) e++;
         int end = q + 1;
-        while (end < nTasks && end - q < (32 >> e) && Lanes(tasks[order[end]].size(), best) == g) end++;
+        while (end < q1 && end - q < (32 >> e) && Lanes(L.tasks[order[end]].size(), best) == g) end++;
         const int share = kSoloRounds << e;
-        bundles.push_back({e, std::max(1, (tasks[order[q]].size() + share - 1) / share), q, end});
+        int head = (e << 4) | (isExport ? kSoloExport : 0);
+        for (int t = q; t < end; t++) {
+            const int kind = L.tasks[order[t]].kind;
+            head |= kind == kSoloDiag ? kSoloHasDiag : kind == kSoloBack ? kSoloIsBack : 0;
+        }
+        bundles.push_back({&L, q, end, e, std::max(1, (longestHere + share - 1) / share), head, 0});
         q = end;
     }
     std::stable_sort(bundles.begin(), bundles.end(), [](const Bundle& a, const Bundle& b) { return a.chunks > b.chunks; });
     // a warp that worked in the level before is the last to be given work: another one has its next chunk at hand already
-    std::vector<int64_t> load(W, 0);
+    int64_t load[kSoloWarps];
     for (int w = 0; w < W; w++) load[w] = warps[w].worked ? kBundleCycles : 0;
     for (Stream& s : warps) s.worked = false;
     for (const Bundle& b : bundles) {
-        const int w = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+        const int w = (int)(std::min_element(load, load + W) - load);
         load[w] += kBundleCycles + b.chunks * kChunkCycles;
         warps[w].worked = true;
-        int32_t head = (b.lg << 4) | (isExport ? kSoloExport : 0);
-        for (int q = b.t0; q < b.t1; q++)
-            head |= tasks[order[q]].kind == kSoloDiag ? kSoloHasDiag : tasks[order[q]].kind == kSoloBack ? kSoloIsBack : 0;
-        std::vector<int32_t>& out = warps[w].chunks;
-        size_t at = out.size();
-        out.resize(at + (size_t)b.chunks * kSoloWords);
-        const int none = isExport ? -1 : 8 * (P.zero + 1);  // where a lane without a result stores
-        for (int k = 0; k < b.chunks; k++)
-            for (int r = 0; r < kSoloRounds; r++)
-                for (int lane = 0; lane < 32; lane++, at += 4) {
-                    const int q = b.t0 + (lane >> b.lg), j = lane & ((1 << b.lg) - 1);
-                    const Task* t = q < b.t1 ? &tasks[order[q]] : nullptr;
-                    const int x = t ? t->p0 + j + ((k * kSoloRounds + r) << b.lg) : 0;
-                    const SoloPair p = t && x < t->p1 ? pairs[x] : SoloPair{P.zero, P.zero, P.one};
-                    const int pivot = 8 * (P.pivots + (t ? t->node : P.one));
-                    int extra;
-                    if (r == 0) extra = 8 * (t && !isExport ? t->out : P.zero);  // an export starts from the zero
-                    else if (r == 1) extra = !t || j > 0 ? none : t->kind == kSoloDiag ? pivot : isExport ? t->out : 8 * t->out;
-                    else if (r == 2) extra = (t && j == 0 ? t->kind : kSoloNone) | head | (k + 1 == b.chunks ? kSoloLast : 0);
-                    else extra = pivot;
-                    int32_t* o = out.data() + at;
-                    o[0] = 8 * p.a;
-                    o[1] = 8 * p.c;
-                    o[2] = 8 * (P.pivots + p.j);
-                    o[3] = extra;
-                }
+        warps[w].bundles.push_back(b);
+        warps[w].chunks += b.chunks;
     }
     for (Stream& s : warps) s.barrier();
 }
 
+// A bundle's chunks as the kernel reads them.
+int32_t* Write(const Place& P, const Bundle& b, int32_t* out) {
+    const bool isExport = (b.head & kSoloExport) != 0;
+    const int zero = 8 * P.zero, one = 8 * (P.pivots + P.one), g = 1 << b.lg;
+    const int none = isExport ? -1 : 8 * (P.zero + 1);  // where a lane without a result stores
+    for (int lane = 0; lane < 32; lane++) {
+        const int q = b.t0 + (lane >> b.lg), j = lane & (g - 1);
+        const Task* t = q < b.t1 ? &b.list->tasks[b.list->order[q]] : nullptr;
+        const int pivot = t ? 8 * (P.pivots + t->node) : one;
+        const int from = t && !isExport ? 8 * t->out : zero;  // an export starts from the zero
+        const int to = !t || j > 0 ? none : t->kind == kSoloDiag ? pivot : isExport ? t->out : 8 * t->out;
+        const int head = (t && j == 0 ? t->kind : kSoloNone) | b.head;
+        const SoloPair *p = t ? b.list->pairs.data() + t->p0 + j : nullptr, *end = t ? b.list->pairs.data() + t->p1 : nullptr;
+        int left = t ? (int)(end - p + g - 1) / g : 0;  // this lane's pairs
+        int32_t* o = out + 4 * lane;
+        for (int k = 0; k < b.chunks; k++) {
+            const int32_t extra[4] = {from, to, k + 1 == b.chunks ? head | kSoloLast | b.bars << 12 : head, pivot};
+            for (int r = 0; r < kSoloRounds; r++, o += 4 * 32) {
+                if (left-- > 0) {
+                    o[0] = 8 * p->a;
+                    o[1] = 8 * p->c;
+                    o[2] = 8 * (P.pivots + p->j);
+                    p += g;
+                } else {
+                    o[0] = o[1] = zero;
+                    o[2] = one;
+                }
+                o[3] = extra[r];
+            }
+        }
+    }
+    return out + (size_t)b.chunks * kSoloWords;
+}
+static_assert(kSoloRounds == 4, "a round carries one of the four further words");
+
 // The levels of a task list, ascending by level number.
-void AddLevels(const Place& P, std::vector<Stream>& warps, TaskList& L) {
-    std::stable_sort(L.tasks.begin(), L.tasks.end(), [](const Task& a, const Task& b) { return a.level < b.level; });
-    for (size_t q = 0; q < L.tasks.size();) {
-        size_t e = q + 1;
-        while (e < L.tasks.size() && L.tasks[e].level == L.tasks[q].level) e++;
-        AddLevel(P, warps, L.pairs.data(), L.tasks.data() + q, (int)(e - q));
-        q = e;
+void AddLevels(std::vector<Stream>& warps, TaskList& L) {
+    const int n = (int)L.tasks.size();
+    if (n == 0) return;
+    int lo = L.tasks[0].level, hi = lo;
+    for (const Task& t : L.tasks) { lo = std::min(lo, t.level); hi = std::max(hi, t.level); }
+    std::vector<int> ptr(hi - lo + 2, 0), byLevel(n);
+    for (const Task& t : L.tasks) ptr[t.level - lo + 1]++;
+    for (int l = 0; l <= hi - lo; l++) ptr[l + 1] += ptr[l];
+    std::vector<int> at(ptr.begin(), ptr.end() - 1);
+    for (int q = 0; q < n; q++) byLevel[at[L.tasks[q].level - lo]++] = q;
+    L.order.reserve(n);
+    for (int l = 0; l <= hi - lo; l++) {
+        if (ptr[l] == ptr[l + 1]) continue;
+        L.order.insert(L.order.end(), byLevel.begin() + ptr[l], byLevel.begin() + ptr[l + 1]);
+        AddLevel(warps, L, ptr[l]);
     }
 }
 
-void Emit(const std::vector<Stream>& warps, std::vector<int32_t>& chunks, std::vector<int32_t>& first) {
+size_t Words(const std::vector<Stream>& warps) {
+    size_t n = 0;
+    for (const Stream& s : warps) n += (size_t)s.chunks * kSoloWords;
+    return n;
+}
+
+// The warps' streams behind what `chunks` holds (which has room for them).
+void Emit(const Place& P, const std::vector<Stream>& warps, std::vector<int32_t>& chunks, std::vector<int32_t>& first) {
+    size_t at = chunks.size();
+    chunks.resize(at + Words(warps));
     for (const Stream& st : warps) {
-        first.push_back((int)(chunks.size() / kSoloWords));
-        first.push_back((int)(st.chunks.size() / kSoloWords));
+        first.push_back((int)(at / kSoloWords));
+        first.push_back(st.chunks);
         first.push_back(st.before);
-        chunks.insert(chunks.end(), st.chunks.begin(), st.chunks.end());
+        int32_t* out = chunks.data() + at;
+        for (const Bundle& b : st.bundles) out = Write(P, b, out);
+        at += (size_t)st.chunks * kSoloWords;
     }
 }
 
@@ -168,6 +214,8 @@ SoloProgram BuildSolo(const Symbolic& s) {
     const Place at{P.zero, P.nVal, P.one};
     std::vector<Stream> warps(kSoloWarps);
     TaskList L;
+    L.tasks.reserve(s.entSlot.size() + s.m);
+    L.pairs.reserve(s.pairs.size() / 2 + s.nnzLU / 2);
     for (size_t e = 0; e < s.entSlot.size(); e++) {
         const bool fwd = s.entKind[e] == kFwd;
         const int k = s.entNode[e], kind = s.entKind[e] == kDiag ? kSoloDiag : kSoloEntry;
@@ -177,14 +225,16 @@ SoloProgram BuildSolo(const Symbolic& s) {
             const int a = s.pairs[2 * q], c = s.pairs[2 * q + 1];
             L.pair(a, fwd ? P.yBase + c : c, nodeOf[a]);
         }
+        L.end();
     }
     for (int k = 0; k < s.m; k++) {  // the backward levels after the others, from the top down
         L.begin(P.yBase + k, kSoloBack, k, 2 * s.nLevels - s.level[k]);
         for (int j = 0; j < s.luCnt[k]; j++) L.pair((int)s.luBase[k] + 1 + j, P.yBase + s.pRows[s.pRowPtr[k] + j], P.one);
+        L.end();
     }
-    AddLevels(at, warps, L);
+    AddLevels(warps, L);
     P.levels = s.nLevels;
-    Emit(warps, P.chunks, P.first);
+    Emit(at, warps, P.chunks, P.first);
     P.on = true;
     return P;
 }
@@ -193,31 +243,21 @@ SoloProgram BuildSolo(const Symbolic& s) {
 
 namespace {
 
+// What the cut is chosen by, per node and per subtree: values held and work.
+struct Tree {
+    std::vector<int64_t> size, weight, subSize, subWeight;
+    std::vector<std::vector<int>> kids;
+    std::vector<int> roots;
+    int64_t total = 0;  // work
+};
+
 // part: a subtree is dealt out whole once it is at most 1 / part of a block's even share of the work
-bool BuildSharedOn(const Symbolic& s, int C, double part, SharedProgram& P) {
+bool BuildSharedOn(const Symbolic& s, const Tree& tree, int C, int cap, double part, SharedProgram& P) {
     const int m = s.m;
-    // values a block can hold, some kept for the zero, the scratch and the solution entries it reads of higher tiers
-    const int cap = (int)((kSoloSmemMax - SoloSmem(0, 0)) / 8) - 1024;
-    std::vector<int64_t> size(m), weight(m, 0), subSize(m, 0), subWeight(m, 0);
-    for (int k = 0; k < m; k++) size[k] = 2 * s.luCnt[k] + 3;
-    for (size_t e = 0; e < s.entSlot.size(); e++) weight[s.entNode[e]] += s.entPairPtr[e + 1] - s.entPairPtr[e] + 4;
-    std::vector<std::vector<int>> kids(m);
-    std::vector<int> heap;
-    int64_t total = 0, all = 0;
-    for (int k = 0; k < m; k++) {
-        subSize[k] += size[k];
-        subWeight[k] += weight[k];
-        total += weight[k];
-        all += size[k];
-        if (s.parent[k] >= 0) {
-            kids[s.parent[k]].push_back(k);
-            subSize[s.parent[k]] += subSize[k];
-            subWeight[s.parent[k]] += subWeight[k];
-        } else {
-            heap.push_back(k);
-        }
-    }
-    if (all > (int64_t)C * cap) return false;
+    const std::vector<int64_t>&size = tree.size, &weight = tree.weight, &subSize = tree.subSize, &subWeight = tree.subWeight;
+    const std::vector<std::vector<int>>& kids = tree.kids;
+    const int64_t total = tree.total;
+    std::vector<int> heap = tree.roots;
     // the tiers above 0: the heaviest subtrees' roots, until the rest can be dealt out evenly; the first of them, as many
     // as block 0 holds, are the last tier
     std::vector<char> tier(m, 0);
@@ -328,8 +368,7 @@ bool BuildSharedOn(const Symbolic& s, int C, double part, SharedProgram& P) {
     // ---- sums towards entries of higher tiers in other blocks ----
     std::vector<TaskList> exports((size_t)C * T);
     {
-        std::vector<std::vector<std::pair<int, SoloPair>>> of((size_t)C * T);  // scratch: pairs by block and tier of their node
-        struct Import { int block, tier, at, e; };
+        std::vector<std::vector<SoloPair>> of((size_t)C * T);  // scratch: pairs by block and tier of their node
         std::vector<int> touched;
         for (size_t e = 0; e < s.entSlot.size(); e++) {
             const int k = s.entNode[e];
@@ -341,7 +380,7 @@ bool BuildSharedOn(const Symbolic& s, int C, double part, SharedProgram& P) {
                 if (cta[j] == cta[k]) continue;
                 const int b = cta[j] * T + tier[j];
                 if (of[b].empty()) touched.push_back(b);
-                of[b].push_back({0, {luAt[a], fwd ? yAt[c] : luAt[c], dAt[j]}});
+                of[b].push_back({luAt[a], fwd ? yAt[c] : luAt[c], dAt[j]});
             }
             if (touched.empty()) continue;
             SharedTier& t = P.blocks[cta[k]].tier[tier[k]];
@@ -350,7 +389,8 @@ bool BuildSharedOn(const Symbolic& s, int C, double part, SharedProgram& P) {
             std::sort(touched.begin(), touched.end());
             for (int b : touched) {
                 exports[b].begin(P.nExport, kSoloEntry, place[b / T].one, 0);
-                for (auto& p : of[b]) exports[b].pair(p.second.a, p.second.c, p.second.j);
+                for (const SoloPair& p : of[b]) exports[b].pair(p.a, p.c, p.j);
+                exports[b].end();
                 of[b].clear();
                 t.importIdx.push_back(P.nExport++);
             }
@@ -375,6 +415,7 @@ bool BuildSharedOn(const Symbolic& s, int C, double part, SharedProgram& P) {
                     const int a = s.pairs[2 * x], c = s.pairs[2 * x + 1], j = nodeOf[a];
                     if (cta[j] == q) D.pair(luAt[a], fwd ? yAt[c] : luAt[c], dAt[j]);
                 }
+                D.end();
                 if (kind == kSoloEntry && D.tasks.back().size() == 0) D.drop();  // it keeps its matrix value and imports
             }
             TaskList& U = up[tier[k]];
@@ -383,15 +424,23 @@ bool BuildSharedOn(const Symbolic& s, int C, double part, SharedProgram& P) {
                 const int r = s.pRows[s.pRowPtr[k] + j];
                 U.pair(luAt[s.luBase[k] + 1 + j], cta[r] == q ? yAt[r] : ghost[q][upIdx[r]], place[q].one);
             }
+            U.end();
         }
+        std::vector<std::vector<Stream>> d(T, std::vector<Stream>(kSoloWarps)), u(d);
+        size_t words = 0;
         for (int t = 0; t < T; t++) {
-            std::vector<Stream> d(kSoloWarps), u(kSoloWarps);
-            AddLevels(place[q], d, down[t]);
-            const TaskList& X = exports[(size_t)q * T + t];
-            if (!X.tasks.empty()) AddLevel(place[q], d, X.pairs.data(), X.tasks.data(), (int)X.tasks.size(), true);
-            Emit(d, B.chunks, B.tier[t].down);
-            AddLevels(place[q], u, up[t]);
-            Emit(u, B.chunks, B.tier[t].up);
+            AddLevels(d[t], down[t]);
+            TaskList& X = exports[(size_t)q * T + t];
+            X.order.resize(X.tasks.size());
+            for (size_t x = 0; x < X.order.size(); x++) X.order[x] = (int)x;
+            if (!X.tasks.empty()) AddLevel(d[t], X, 0, true);
+            AddLevels(u[t], up[t]);
+            words += Words(d[t]) + Words(u[t]);
+        }
+        B.chunks.reserve(words);
+        for (int t = 0; t < T; t++) {
+            Emit(place[q], d[t], B.chunks, B.tier[t].down);
+            Emit(place[q], u[t], B.chunks, B.tier[t].up);
         }
     };
     std::atomic<int> next{0};
@@ -408,10 +457,30 @@ bool BuildSharedOn(const Symbolic& s, int C, double part, SharedProgram& P) {
 }  // namespace
 
 SharedProgram BuildShared(const Symbolic& s) {
+    // values a block can hold, some kept for the zero, the scratch and the solution entries it reads of higher tiers
+    const int cap = (int)((kSoloSmemMax - SoloSmem(0, 0)) / 8) - 1024;
+    const int m = s.m;
+    const int64_t all = s.nnzLU + 2 * (int64_t)m;
+    if (m <= 0 || all > 16 * (int64_t)cap) return SharedProgram();
+    Tree t;
+    t.size.resize(m);
+    t.weight.assign(m, 0);
+    t.kids.resize(m);
+    for (int k = 0; k < m; k++) t.size[k] = 2 * s.luCnt[k] + 3;
+    for (size_t e = 0; e < s.entSlot.size(); e++) t.weight[s.entNode[e]] += s.entPairPtr[e + 1] - s.entPairPtr[e] + 4;
+    t.subSize = t.size;
+    t.subWeight = t.weight;
+    for (int k = 0; k < m; k++) {  // parents have higher steps
+        t.total += t.weight[k];
+        if (s.parent[k] < 0) { t.roots.push_back(k); continue; }
+        t.kids[s.parent[k]].push_back(k);
+        t.subSize[s.parent[k]] += t.subSize[k];
+        t.subWeight[s.parent[k]] += t.subWeight[k];
+    }
     for (int C : {2, 4, 8, 16})
         for (double part : {2.0, 1.5, 1.0}) {
             SharedProgram P;
-            if (s.m > 0 && BuildSharedOn(s, C, part, P)) return P;
+            if (all <= (int64_t)C * cap && BuildSharedOn(s, t, C, cap, part, P)) return P;
         }
     return SharedProgram();
 }
