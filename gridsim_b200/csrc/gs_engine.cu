@@ -1925,7 +1925,7 @@ struct gs_grid {
     int splitB = 0;     // first level run by the persistent kernels in the triangular solves
     gs::DevSolo solo{};  // one block's shared-memory program of the grid, where its factors fit (on)
     gs::DevShared shared{};  // a cluster's program, where the factors fit one but not a block (on)
-    gs::DevBuf sharedScratch; // its exports and upper solutions (calls on the context's stream)
+    gs::DevBuf sharedScratch; // its exports and upper solutions (calls on the context's stream), sized with the workspace
     gs::DevBuf soloNext; // its system counter and step maximum (calls on the context's stream)
     int tailSplit = 0;  // first level the few-systems path runs as one CTA per system
     int tailMax = gs::kTailMaxSystems;  // the few-systems path takes over at this many systems still stepping
@@ -2278,6 +2278,8 @@ int UploadGrid(gs_grid* G) {
     return GS_OK;
 }
 
+constexpr int kSharedSystemBlocks = 4096;  // the most systems x blocks^2 that go to the clusters' program (SharedTakes)
+
 size_t PerSystemBytes(const Symbolic& s, int precision) {
     size_t t = precision == GS_PREC_MIXED ? 4 : 8;
     size_t refine = precision == GS_PREC_MIXED ? (size_t)s.m * (t + 8) : 0;
@@ -2336,6 +2338,12 @@ int EnsureWorkspace(gs_grid* G, int B, int precision, bool classify, bool loadSc
     (void)precision;
     int rc = EnsureWs(G->ctx, G->sym, G->tws, cap, GS_PREC_FP64, 0, loadScale);
     if (rc != GS_OK) return rc;
+    // the clusters' exports, for the most systems that go there at once: no allocation between two steps
+    if (const DevShared& P = G->shared; P.on) {
+        gs_ctx* ctx = G->ctx;
+        const size_t most = std::min({B, G->tailMax, kSharedSystemBlocks / (P.ctas * P.ctas)});
+        GS_CUDA(G->sharedScratch.alloc(most * (P.nExport + P.nUpper) * sizeof(double)));
+    }
     return EnsureWs(G->ctx, G->sym, G->ws, B, precision, classify ? G->sym.nbr + G->host.nBnd + G->sym.n : 0,
                     loadScale);
 }
@@ -2526,7 +2534,7 @@ bool SoloTakes(const gs_grid* G, int count, bool mixed) {
 // 148 4.6 / 5.1, 296 8.1 / 9.2; 4,000 (8 blocks) 9 2.0 / 7.2, 74 8.1 / 8.5, 148 15.3 / 10.7; one step at 10,000 (16
 // blocks) 6 0.61 / 1.39, 9 1.19 / 2.70, 29 3.2 / 2.0.
 bool SharedTakes(const gs_grid* G, int n) {
-    return G->shared.on && (int64_t)n * G->shared.ctas * G->shared.ctas <= 4096;
+    return G->shared.on && (int64_t)n * G->shared.ctas * G->shared.ctas <= kSharedSystemBlocks;
 }
 
 // The linear solves of the listed systems of b (FP64) on clusters.
