@@ -79,11 +79,10 @@ __device__ __forceinline__ bool zipLoad(const DevGrid& g, int i, double vm, doub
 //    replaced by their reduced values), the mismatch into the right-hand side (and its FP64 copy in mixed
 //    precision), the Jacobian blocks of row i into their LU slots; folds |mismatch| into localMax and sets bad
 //    (1: mismatch not finite, 2: Jacobian not finite).
-// OWN: lu and y are one system's own, not interleaved (k_solo). LG lanes share a bus (aligned groups of a warp, all of them here together): its cells dealt to them in turn, the sums
-// completed over the group; the first lane does the rest.
+// OWN: lu and y are one system's own, not interleaved (k_solo). LG lanes share a bus (aligned groups of a warp, all of
+// them here together): its cells dealt to them in turn, the sums completed over the group; the first lane does the rest.
 template <typename T, int LG = 1, bool OWN = false>
-__device__ __forceinline__ void busMismatchJac(const DevGrid& g, const DevBatch& b, int i, int s, int fillJac, double* pOut,
-                                               double* qOut, double& localMax, int& bad) {
+__device__ __forceinline__ void busMismatchJac(const DevGrid& g, const DevBatch& b, int i, int s, double& localMax, int& bad) {
     const int gl = LG == 1 ? 0 : (int)(threadIdx.x & (LG - 1));
     const size_t B = (size_t)b.B;
     const double vmi = b.vm[i * B + s], vai = b.va[i * B + s];
@@ -96,7 +95,7 @@ __device__ __forceinline__ void busMismatchJac(const DevGrid& g, const DevBatch&
     const bool pId = g.qlim && (et == 3 || et == 0);
     const bool qId = g.qlim && et != 1;
     const int kp = g.busP[i], kq = g.busQ[i];
-    const bool fill = fillJac && (kp >= 0 || kq >= 0);
+    const bool fill = kp >= 0 || kq >= 0;
     const size_t K = OWN ? 1 : B;  // the Jacobian and right-hand side: interleaved, or this system's own arrays
     const size_t so = OWN ? 0 : s;
     T* lu = (T*)b.lu;
@@ -160,7 +159,6 @@ __device__ __forceinline__ void busMismatchJac(const DevGrid& g, const DevBatch&
         if (sl.w >= 0) lu[sl.w * K + so] = (T)L;
         bad |= (isfinite(H) && isfinite(N) && isfinite(M) && isfinite(L)) ? 0 : 2;
     }
-    if (pOut) { pOut[i * B + s] = P; qOut[i * B + s] = Q; }
     double pspec = b.loadScale ? g.pgen[i] - sc * g.pload[i] : g.pgen[i] - g.pload[i];
     double qspec = b.loadScale ? g.qgen[i] - sc * g.qload[i] : g.qgen[i] - g.qload[i];
     if (b.specBus && b.specBus[s] == i) {  // a generator outage: the bus loses the unit's output
@@ -196,17 +194,14 @@ __device__ __forceinline__ void busMismatchJac(const DevGrid& g, const DevBatch&
 
 // The batched kernel. Block (32, 8): lane = system, y = bus within the block.
 template <typename T>
-__global__ void __launch_bounds__(256) k_mismatch_jac(DevGrid g, DevBatch b, int fillJac, double* pOut, double* qOut,
-                                                      const int* list, int nList) {
+__global__ void __launch_bounds__(256) k_mismatch_jac(DevGrid g, DevBatch b, const int* list, int nList) {
     const int lane = threadIdx.x, w = threadIdx.y;
     const int s = sysAt(blockIdx.y * 32 + lane, list, nList);
     const int i = blockIdx.x * 8 + w;
     double localMax = 0.0;
     int bad = 0;  // 1: mismatch not finite, 2: Jacobian not finite
     const bool live = i < g.n && s >= 0 && s < b.count && b.active[s];
-    if (live) {
-        busMismatchJac<T>(g, b, i, s, fillJac, pOut, qOut, localMax, bad);
-    }
+    if (live) busMismatchJac<T>(g, b, i, s, localMax, bad);
     __shared__ double red[8][32];
     __shared__ int redBad[8][32];
     red[w][lane] = localMax;
@@ -1664,7 +1659,6 @@ __global__ void k_compact(DevGrid g, DevBatch b, Classify c, const int* first, i
     }
 }
 
-// Line flows of system 0 (single solve result).
 // rows[k * n + i] (a system a row) into the batch's interleaved[i * B + k] and back times f; systems past cnt are 1.
 // Tiles of 32 x 32 through shared memory, so that both sides move whole lines: grid (ceil(n / 32), ceil(B / 32)), block
 // (32, 8). The host's own transposition of the load scales and states of 777 systems of 2,750 buses took half the call.
@@ -2252,7 +2246,7 @@ int UploadGrid(gs_grid* G) {
         const int32_t* chunks = nullptr;
         if ((rc = Upload(G, S.chunks, &chunks)) != GS_OK || (rc = Upload(G, S.first, &d.first)) != GS_OK) return rc;
         d.chunks = reinterpret_cast<const int4*>(chunks);
-        d.m = S.m; d.nVal = S.nVal; d.yBase = S.yBase; d.zero = S.zero; d.one = S.one;
+        d.m = S.m; d.nVal = S.nVal; d.yBase = S.yBase; d.one = S.one;
         d.on = 1;
     }
     G->shared.on = 0;
@@ -2532,7 +2526,9 @@ bool SoloTakes(const gs_grid* G, int count, bool mixed) {
 // system alone, so more waves of clusters soon cost more than the walk with its smaller share of blocks a system. Measured
 // (whole solve_batch of 4 to 5 steps, ms, this / the walk): 2,000 buses (4 blocks) 1 system 1.1 / 2.4, 37 2.1 / 5.1,
 // 148 4.6 / 5.1, 296 8.1 / 9.2; 4,000 (8 blocks) 9 2.0 / 7.2, 74 8.1 / 8.5, 148 15.3 / 10.7; one step at 10,000 (16
-// blocks) 6 0.61 / 1.39, 9 1.19 / 2.70, 29 3.2 / 2.0.
+// blocks) 6 0.61 / 1.39, 9 1.19 / 2.70, 29 3.2 / 2.0. Batches on other grids: 1,000 buses (2 blocks, never past the line)
+// 37 0.90 / 3.0, 296 2.25 / 4.3; 10,000 buses, systems that run to the cap of 20 steps, 12 16.2 / 31.5, 16 20 / 35; 8,000 (16
+// blocks) 64 55 / 42.
 bool SharedTakes(const gs_grid* G, int n) {
     return G->shared.on && (int64_t)n * G->shared.ctas * G->shared.ctas <= kSharedSystemBlocks;
 }
@@ -2807,10 +2803,9 @@ int Newton(gs_grid* G, int count, bool useScale, bool startFromWs, const gs_pf_o
     for (int iter = 0; iter <= maxLoop; iter++) {
         if (timed) cudaEventRecord(ev[0], st);
         if (listCount > 0)
-            k_mismatch_jac<double><<<dim3(nodeBlocks.x, (listCount + 31) / 32), blk8, 0, st>>>(g, cur, 1, nullptr, nullptr,
-                                                                                       cur.activeList, listCount);
+            k_mismatch_jac<double><<<dim3(nodeBlocks.x, (listCount + 31) / 32), blk8, 0, st>>>(g, cur, cur.activeList, listCount);
         else
-            k_mismatch_jac<T><<<dim3(nodeBlocks.x, cur.B / 32), blk8, 0, st>>>(g, cur, 1, nullptr, nullptr, nullptr, 0);
+            k_mismatch_jac<T><<<dim3(nodeBlocks.x, cur.B / 32), blk8, 0, st>>>(g, cur, nullptr, 0);
         if (timed) cudaEventRecord(ev[1], st);
         cudaMemsetAsync(cur.activeCount, 0, 2 * sizeof(int), st);
         if (g.qlim) {
@@ -2854,7 +2849,7 @@ int Newton(gs_grid* G, int count, bool useScale, bool startFromWs, const gs_pf_o
                 k_gather<<<dim3(nodeBlocks.x, stride / 32), blk8, 0, st>>>(b, cur, G->tws.origin.as<int>(), s.n);
                 // this iteration's Jacobian and right-hand side, rebuilt in the compact workspace; the mismatch
                 // maximum it records was already taken by k_status
-                k_mismatch_jac<double><<<dim3(nodeBlocks.x, stride / 32), blk8, 0, st>>>(g, cur, 1, nullptr, nullptr, nullptr, 0);
+                k_mismatch_jac<double><<<dim3(nodeBlocks.x, stride / 32), blk8, 0, st>>>(g, cur, nullptr, 0);
                 cudaMemsetAsync(cur.maxMis, 0, (size_t)nActive * sizeof(unsigned long long), st);
                 launches += 3;
                 compacted = true;
@@ -2923,7 +2918,7 @@ int Newton(gs_grid* G, int count, bool useScale, bool startFromWs, const gs_pf_o
                 k_gather<<<dim3(nodeBlocks.x, B2 / 32), blk8, 0, st>>>(b, mid, G->mws.origin.as<int>(), s.n);
                 // this iteration's Jacobian and right-hand side, rebuilt in the mid workspace; the mismatch maximum it
                 // records was already taken by k_status
-                k_mismatch_jac<T><<<dim3(nodeBlocks.x, B2 / 32), blk8, 0, st>>>(g, mid, 1, nullptr, nullptr, nullptr, 0);
+                k_mismatch_jac<T><<<dim3(nodeBlocks.x, B2 / 32), blk8, 0, st>>>(g, mid, nullptr, 0);
                 cudaMemsetAsync(mid.maxMis, 0, (size_t)nActive * sizeof(unsigned long long), st);
                 launches += 3;
                 cur = mid;

@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(1024) k_newton(const DevGrid* grids, const Mul
         for (int iter = 0;; iter++) {
             double lm = 0.0;
             int bad = 0;
-            for (int i = tid; i < n; i += bd) busMismatchJac<T>(g, b, i, 0, 1, nullptr, nullptr, lm, bad);
+            for (int i = tid; i < n; i += bd) busMismatchJac<T>(g, b, i, 0, lm, bad);
             lm = blockMaxD(lm, redD);
             bad = blockOrI(bad, redI);
             if (tid == 0) {

@@ -248,7 +248,7 @@ cudaError_t LaunchA(gs_server* S, Lane& L) {
     }
     cudaMemsetAsync(b.activeCount, 0, 2 * sizeof(int), L.st);
     cudaMemsetAsync(L.doneD.p, 0, sizeof(int), L.st);
-    k_mismatch_jac<T><<<dim3((g.n + 7) / 8, L.C / 32), blk8, 0, L.st>>>(g, b, 1, nullptr, nullptr, nullptr, 0);
+    k_mismatch_jac<T><<<dim3((g.n + 7) / 8, L.C / 32), blk8, 0, L.st>>>(g, b, nullptr, 0);
     k_status_each<<<(L.C + 255) / 256, 256, 0, L.st>>>(b, o.tolerance, o.diverge_limit_pu, o.max_iterations, L.doneD.as<int>());
     cudaMemcpyAsync(L.hCounts.p, b.activeCount, 2 * sizeof(int), cudaMemcpyDeviceToHost, L.st);
     cudaMemcpyAsync(L.hDone.p, L.doneD.p, (size_t)(1 + L.C) * sizeof(int), cudaMemcpyDeviceToHost, L.st);

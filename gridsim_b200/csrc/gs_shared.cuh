@@ -1,6 +1,6 @@
 // gs_shared.cuh — the linear solve of a few systems whose factors fit the shared memory of a cluster (SharedProgram),
-// sm_100a: one cluster a system, every block's part of the tree walked with block barriers only, the cluster meeting three
-// to five times (between tiers).
+// sm_100a: one cluster a system, every block's part of the tree walked with block barriers only, the cluster meeting
+// between tiers only: twice with two tiers, four times with three.
 //
 // The walk over L2 (gs_cluster.cuh) meets at a cluster barrier twice per elimination level and loads every operand from
 // L2. Here the operands are in the block's own shared memory; what crosses blocks is the sums of the subtrees towards the

@@ -202,7 +202,7 @@ void Emit(const Place& P, const std::vector<Stream>& warps, std::vector<int32_t>
 SoloProgram BuildSolo(const Symbolic& s) {
     SoloProgram P;
     const int64_t values = s.nnzLU + s.m + 2;
-    if (s.m <= 0 || values > 65535 || SoloSmem(values, s.m) > kSoloSmemMax) return P;
+    if (s.m <= 0 || SoloSmem(values, s.m) > kSoloSmemMax) return P;
     P.m = s.m;
     P.nVal = (int)values;
     P.yBase = (int)s.nnzLU;

@@ -36,7 +36,7 @@ __device__ __forceinline__ int blockOrI(int v, int* red) {
 
 // SoloProgram on the device.
 struct DevSolo {
-    int on, m, nVal, yBase, zero, one;
+    int on, m, nVal, yBase, one;
     const int4* chunks;
     const int* first;
 };
@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(kSoloThreads, 2) k_solo(DevGrid g, DevSolo P, 
             __syncthreads();
             double mx = 0.0;
             int bad = 0;
-            for (int q = tid; q < 2 * n; q += bd) busMismatchJac<double, 2, true>(g, o, q >> 1, s, 1, nullptr, nullptr, mx, bad);
+            for (int q = tid; q < 2 * n; q += bd) busMismatchJac<double, 2, true>(g, o, q >> 1, s, mx, bad);
             mx = blockMaxD(mx, redD);
             bad = blockOrI(bad, redI);
             if (tid == 0) {

@@ -45,7 +45,7 @@ class PowerFlowOptions:
     precision: str = "fp64"          # "fp64" or "mixed" (FP32 LU and solves, FP64 mismatch and update)
     warm_start_from_base: bool = False
     batch_width: int = 0
-    phase_timing: bool = False
+    phase_timing: bool = False       # phases launched and timed one by one, also where a run is one launch otherwise
     post_fault_rating: str = "A"     # "A", "B" or "C": the rating outage states are judged against (screens)
     max_q_limit_passes: int = 100    # MaxQLimitPasses
     revert_q_limits: bool = False    # RevertQLimits

@@ -150,7 +150,9 @@ typedef struct gs_pf_opts {
     int32_t warm_start_from_base;   /* screens: solve the intact grid first and start every outage from
                                        its solution (GridScenario.WithSolvedVoltages, Simulation/GridScenario.cs:35-52) */
     int32_t batch_width;            /* systems per device batch; 0 = choose from free HBM */
-    int32_t phase_timing;           /* 1: time each phase with CUDA events (no graph replay) into the result */
+    int32_t phase_timing;           /* 1: time each phase with CUDA events into the result; the step is then launched phase by
+                                       phase (no graph replay), also on grids whose runs otherwise take one launch that
+                                       holds a system a block: the times are those of the phases' own kernels */
     int32_t post_fault_rating;      /* enum gs_post_fault_rating, screens only; default GS_RATE_A */
     int32_t max_q_limit_passes;     /* cap on PV->PQ switching passes (MaxQLimitPasses); 0 = the default 100 */
     int32_t revert_q_limits;        /* RevertQLimits: a pinned bus may go back to PV within a switching pass; 0 */
