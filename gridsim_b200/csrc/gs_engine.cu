@@ -194,7 +194,7 @@ __device__ __forceinline__ void busMismatchJac(const DevGrid& g, const DevBatch&
 
 // The batched kernel. Block (32, 8): lane = system, y = bus within the block. Bound by the latency of the gathered loads:
 // four blocks an SM (64 registers a thread), since at 72 registers, three blocks, the 5,000-outage screen of the 10,000-bus
-// grid takes 14.5 ms here instead of 11.8.
+// grid takes 14.5 ms here instead of 12.1.
 template <typename T>
 __global__ void __launch_bounds__(256, 4) k_mismatch_jac(DevGrid g, DevBatch b, const int* list, int nList) {
     const int lane = threadIdx.x, w = threadIdx.y;

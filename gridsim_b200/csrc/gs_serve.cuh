@@ -95,7 +95,7 @@ struct Lane {
     bool warm = false;
     // The linear solves run in shared memory, in FP64 whatever the precision asked for: a block's (the grid's k_solo
     // program), or a cluster's while all the slots may go there (SharedTakes). The walk over L2 was bound by its barriers: 256
-    // requests on four grids of 100 to 2,000 buses took 12.2 ms, now 5.2. Decided when the loop starts (PlaceLanes).
+    // requests on four grids of 100 to 2,000 buses took 12.2 ms, now 4.8 to 6.1. Decided when the loop starts (PlaceLanes).
     bool onChip = false, placed = false;
     DevBuf scratch;      // the clusters' exports, for every slot
     std::unique_ptr<Workspace> ws;

@@ -5,7 +5,8 @@
 // mismatch and Jacobian straight into shared memory, the status test (the Q-limit passes too), the linear solve from
 // the program's bundles, the damped update. A level of the solve costs one block barrier, one round of shared-memory
 // operand loads, a short sum and a store; the index data of the next bundle (from L2) is loaded while this one is summed.
-// Bound by that chain: a level takes about 0.15 us.
+// Bound by that chain: a run of a 120-bus grid, 3 steps of 44 levels down and up and 4 mismatch evaluations, takes 78 us, so at
+// most 0.3 us a level.
 #pragma once
 
 namespace gs {
