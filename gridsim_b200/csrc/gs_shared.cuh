@@ -51,8 +51,11 @@ __global__ void __launch_bounds__(kSoloThreads, 1) k_shared(DevGrid g, DevShared
     for (int k = B.nLu + tid; k < nVal; k += kSoloThreads) val[k] = 0.0;
     if (tid == 0) { val[nVal + B.nDinv - 1] = 1.0; sCollapsed = 0; }
     __syncthreads();
-    for (int k = tid; k < B.nY; k += kSoloThreads) val[__ldg(ints + B.yAt + k)] = y[__ldg(ints + B.yNode + k) * S];
-    for (int k = tid; k < B.nDinv - 1; k += kSoloThreads) val[nVal + k] = val[__ldg(ints + B.diagAt + k)];  // for the pivots' floors
+    for (int k = tid; k < B.nY; k += kSoloThreads) {  // a node's right-hand side, and its diagonal for the pivot's floor
+        const int at = __ldg(ints + B.yAt + k), diag = __ldg(ints + B.diagAt + k);
+        val[at] = y[__ldg(ints + B.yNode + k) * S];
+        val[nVal + k] = val[diag];
+    }
     __syncthreads();
     const int4* chunks = P.chunks + B.chunks * (kSoloWords / 4);
     auto meet = [&]() {
